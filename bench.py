@@ -134,19 +134,19 @@ def peaks() -> dict:
 def launches_per_step(n: int) -> int:
     """The library's kernel launches in one headline step (wrs_build + wrs_sample): total mass,
     partition, the split descent (split-pack grids of >= 512 CTAs of 479 subproblems), the
-    split-pack, the coin filter (2^22 < N <= 2^26) and the sampler."""
+    split-pack, the alias blocks (2^22 < N <= 2^27) and the sampler."""
     blocks = -(-(n // SPLIT_SIZE) // 479)
-    return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 26))
+    return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 27))
 
 
 def profiled_traffic(l2_fetch: int) -> float | None:
-    """DRAM bytes of one headline alias-sampling launch (with the tables' coin filters, the
+    """DRAM bytes of one headline alias-sampling launch (through the tables' alias blocks, the
     mean over the three distributions' launches) at the given L2 fetch granularity, from the
-    committed ncu summary (a line `dram_bytes_per_launch_coin_filter[l2=B]: X` per captured
+    committed ncu summary (a line `dram_bytes_per_launch_blocks[l2=B]: X` per captured
     granularity), if it holds that granularity."""
     if not os.path.exists(PROFILE_TRAFFIC):
         return None
-    key = f"dram_bytes_per_launch_coin_filter[l2={l2_fetch}]:"
+    key = f"dram_bytes_per_launch_blocks[l2={l2_fetch}]:"
     for line in open(PROFILE_TRAFFIC):
         if line.strip().startswith(key):
             return float(line.split(":", 1)[1].split()[0])
@@ -555,13 +555,14 @@ def main() -> None:
                 "traffic_l2_fetch": tune["l2_fetch"],
                 "traffic_source": "ncu dram__bytes_read.sum + dram__bytes_write.sum per "
                                   "headline launch (mean of the uniform, Zipf and log-normal "
-                                  "launches, coin filters in use) at this run's L2 fetch "
+                                  "launches, through the alias blocks) at this run's L2 fetch "
                                   "granularity, null where none was captured at it "
                                   "(profiles/alias_sample_n26_s28.md)",
                 "kernel": "k_alias_sample",
-                "bytes_model": "12 B/sample (8 B entry + 4 B index), as without the coin "
-                               "filter; with it the entry is read only where the coin does "
-                               "not decide (plus 1 B of filter from L2)",
+                "bytes_model": "12 B/sample (8 B entry + 4 B index), as by the table "
+                               "alone; through the alias blocks the entry is read only "
+                               "where its block does not decide (plus 32 B of block, mostly "
+                               "from L2)",
                 "peak_source": pk["source"],
                 "sector_model_frac": (36.0 * s / samp_s / 1e9) / pk["hbm_gbs"],
                 "random_gather": {
@@ -1414,10 +1415,10 @@ def kernel_breakdown(W, pkg, wrs, internals, weights, samples, n, s, stream, pea
     rec("alias_sample",
         timed(lambda: wrs.alias_sample(stream, table, n, s, 99, 0, samples)), 12 * s, s,
         "samples")
-    # the same draws through the buffers after a build, i.e. with the table's coin filter
+    # the same draws through the buffers after a build, i.e. through the table's alias blocks
     ab = W.WRSBuffers(w, samples, internals)
     wrs.build(stream, ab, n)
-    rec("alias_sample_coin_filter",
+    rec("alias_sample_blocks",
         timed(lambda: wrs.sample(stream, ab, n, s, seed=99)), 12 * s, s, "samples")
     # serial split-pack (split records + pack from them), the two pack strategies, against the
     # inline split-pack at the same split size

@@ -375,6 +375,7 @@ struct PartArgs {
     const uint32_t* bw_c;
     const float* bw_h;
     const float* bw_l;
+    uint16_t* classes;  // heavy bits, 16 items per word (null: not wanted)
 };
 
 // One CTA = one tile of 4096 weights.  The tile is loaded with 16-byte coalesced loads and
@@ -451,7 +452,7 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
             y[4 * j + 2] = q.z;
             y[4 * j + 3] = q.w;
         }
-        uint32_t tc = 0;
+        uint32_t heavies = 0;  // one bit per heavy item
         float th = 0.f, tl = 0.f;
         ff fh{0.f, 0.f}, fl{0.f, 0.f};
 #pragma unroll
@@ -460,16 +461,22 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
                 // one float-float add on the selected accumulator (the operations of adding to
                 // it in a branch, without the two predicated paths)
                 const bool hv = y[i] > pivot;
-                tc += hv ? 1u : 0u;
+                heavies |= hv ? 1u << i : 0u;
                 const ff acc = ff_add_f(hv ? fh : fl, y[i]);
                 fh = hv ? acc : fh;
                 fl = hv ? fl : acc;
             } else if (y[i] > pivot) {
-                ++tc;
+                heavies |= 1u << i;
                 th = __fadd_rn(th, y[i]);
             } else {
                 tl = __fadd_rn(tl, y[i]);
             }
+        }
+        const uint32_t tc = __popc(heavies);
+        if constexpr (!BATCH && !BW) {
+            if (a.classes)
+                a.classes[static_cast<size_t>(lt) * kTileThreads + threadIdx.x] =
+                    static_cast<uint16_t>(heavies);
         }
         const uint32_t ic = warp_incl_u(tc, lane);
         s_lc[threadIdx.x] = ic - tc;
@@ -729,9 +736,10 @@ static void part_dispatch(cudaStream_t st, uint32_t precision, uint32_t grid, co
 cudaError_t launch_prefix_partition(cudaStream_t st, bool comp, const float* w, uint32_t n,
                                     BuildCtrl* ctrl, PartState* states, uint32_t cap_tiles,
                                     uint32_t* idx_out, float* prefix_out, float* elems_out,
-                                    float* prefix_lo_out) {
-    const PartArgs a{w,         n,           ctrl,          &ctrl->part, states,   cap_tiles,
-                     kSpinLimit, &ctrl->status, idx_out,  prefix_out, elems_out, prefix_lo_out};
+                                    float* prefix_lo_out, uint16_t* classes) {
+    const PartArgs a{w,          n,             ctrl,    &ctrl->part, states,    cap_tiles,
+                     kSpinLimit, &ctrl->status, idx_out, prefix_out,  elems_out, prefix_lo_out,
+                     nullptr,    nullptr,       nullptr, classes};
     const uint32_t precision = prefix_lo_out ? 2u : (comp ? 1u : 0u);
     part_dispatch<false>(st, precision, tiles_for(n), a, BatchView{});
     return cudaGetLastError();

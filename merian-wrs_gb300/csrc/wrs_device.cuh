@@ -429,4 +429,12 @@ __device__ __forceinline__ void ld_u32x8(const uint32_t* p, uint4& a, uint4& b) 
                  : "l"(p));
 }
 
+// an alias block (32 bytes, aligned), kept in L2 rather than the table entries around it
+__device__ __forceinline__ void ld_block(const uint32_t* p, uint4& a, uint4& b) {
+    asm volatile("ld.global.nc.L1::no_allocate.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(a.x), "=r"(a.y), "=r"(a.z), "=r"(a.w), "=r"(b.x), "=r"(b.y), "=r"(b.z),
+                   "=r"(b.w)
+                 : "l"(p));
+}
+
 }  // namespace wrs

@@ -54,7 +54,7 @@ struct alignas(64) BuildCtrl {
     double mean64;       // total / N in FP64
     float mean_lo;       // (float)(mean64 - mean): mean64 as the float-float pair (mean, mean_lo)
     uint32_t pad0;
-    unsigned long long coin_sum;  // sum of the table's coin-filter codes (k_coin_filter)
+    unsigned long long block_reads;  // 8 x the alias blocks' expected entry reads (k_alias_blocks)
     uint32_t pad[12];
 };
 static_assert(sizeof(BuildCtrl) == 128, "BuildCtrl layout");
@@ -147,7 +147,7 @@ cudaError_t launch_total_mass(cudaStream_t st, const float* w, uint32_t n, doubl
 cudaError_t launch_prefix_partition(cudaStream_t st, bool comp, const float* w, uint32_t n,
                                     BuildCtrl* ctrl, PartState* states, uint32_t cap_tiles,
                                     uint32_t* idx_out, float* prefix_out, float* elems_out,
-                                    float* prefix_lo_out);
+                                    float* prefix_lo_out, uint16_t* classes = nullptr);
 // comp: runs k_total_mass first (into `partials`, >= tiles_for(n) doubles) for the grid of the
 // exact carries
 cudaError_t launch_scan(cudaStream_t st, bool comp, const float* in, uint32_t n, float* out,
@@ -190,26 +190,54 @@ cudaError_t launch_split_pack(cudaStream_t st, bool r64, bool full_light, const 
                               const uint32_t* idx, const float* elems, const float* prefix,
                               const float* prefix_lo, const BuildCtrl* ctrl, uint32_t* status,
                               uint32_t n, uint32_t split_size, uint2* table, int2* descent);
-// coins / coin_sum: the table's coin filter and the sum of its codes (k_coin_filter), or
+// A table's alias blocks: per 32 consecutive buckets one 32-byte sector that decides most samples
+// of them without their 8-byte entries, with the same result.  code (three bit planes) is the
+// eighth of [0, 1) each bucket's p lies in: a coin in a lower one is below p and keeps, one in a
+// higher one takes the alias.  The aliases follow from the partition's order, which is stable: a
+// heavy bucket's alias is the next heavy bucket, and the light buckets', in index order, rise and
+// change only from time to time.  `cls` has a bit per heavy bucket, `head` the first light bucket's
+// alias, `sw` a bit per light bucket whose alias differs from the light bucket's before, and `off`
+// the aliases the switches begin: their distances from head, `width` bits each, or their steps
+// (less one) from one to the next as nibbles.  Entries are read for coins in the bucket's own
+// eighth, for a block's last heavy bucket, and in blocks whose aliases are not encoded.
+struct alignas(32) AliasBlock {
+    uint32_t code[3];
+    uint32_t cls;
+    uint32_t head;  // alias (27 bits) | width << 27
+    uint32_t sw;
+    uint32_t off[2];
+};
+static_assert(sizeof(AliasBlock) == 32, "one alias block is one 32-byte sector");
+constexpr uint32_t kAliasHeadBits = 27;
+constexpr uint32_t kAliasHeadMask = (1u << kAliasHeadBits) - 1u;
+// widths that say something else: the aliases are not encoded; `off` holds steps
+constexpr uint32_t kAliasNone = 0, kAliasSteps = 1;
+constexpr int kBlockBuildThreads = 128;
+// samples per thread through the blocks (2^28 samples of uniform weights, n = 2^26: 1.66 ms with 2,
+// 2.00 with 4, whose 32 block words a thread leave 4 CTAs on an SM, 2.24 with 1)
+constexpr int kBlockPerThread = 2;
+__host__ __device__ inline uint32_t alias_blocks_of(uint32_t n) { return (n + 31u) / 32u; }
+// blocks / reads: the table's alias blocks and their expected entry reads (launch_alias_blocks), or
 // nullptr; samples are the same either way
 cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, const uint2* table,
-                                const uint8_t* coins, const unsigned long long* coin_sum,
+                                const AliasBlock* blocks, const unsigned long long* reads,
                                 uint32_t n, uint64_t s, uint64_t seed, uint64_t offset,
                                 uint32_t* out);
-// the filter and, into *coin_sum (zeroed first, on the stream), the sum of its codes
-cudaError_t launch_coin_filter(cudaStream_t st, const uint2* table, uint32_t n, uint8_t* coins,
-                               unsigned long long* coin_sum);
-// Tables of kCoinMinN < n <= kCoinMaxN weights get a coin filter (n bytes): a smaller table
-// stays in L2 by itself, and a larger filter would not.  The sampler consults it when the
-// codes average at least kCoinMinMean (out of 255): then at most ~78 % of the samples read
-// their entry.  Measured at N = 2^26 on a box whose plain sampler takes 5.13 ms for 2^28
-// samples, the filtered one took 0.66 + 5.45 f ms with f the share of samples reading their
-// entry (f = 0.42 uniform, 0.75 log-normal(0, 2), 0.88 Zipf(1.1): 2.94 / 4.77 / 5.59 ms); on a
-// box whose plain sampler takes 3.77 ms the uniform table took 2.56 ms and the log-normal one
-// 4.06 ms, so tables near the threshold gain on the one and lose on the other.
-constexpr uint32_t kCoinMinN = 1u << 22;
-constexpr uint32_t kCoinMaxN = 1u << 26;
-constexpr uint64_t kCoinMinMean = 56;
+// the blocks of table[0, n) and, into *reads (zeroed first, on the stream), 8 times the entry
+// reads one sample of every bucket would cost; classes: the partition's heavy bits
+cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint32_t* classes,
+                                uint32_t n, AliasBlock* blocks, unsigned long long* reads);
+// Tables of kBlockMinN < n <= kBlockMaxN weights get alias blocks.  Through the blocks a sample
+// costs its 32-byte sector and the decoding (190 G samples/s while the blocks stay in L2); by the
+// table alone it costs its 8-byte entry, 250 G/s from L2 and 50 G/s from HBM.  2^26 samples of
+// uniform weights, us, by the table / through the blocks: n = 4.0 M 274 / 352, 6.0 M 423 / 353,
+// 8.0 M 549 / 353, 12 M 749 / 355; 2^28 samples: n = 2^26 5300 / 1640, 2^27 (blocks of 128 MB, half of
+// them in L2) 5508 / 3064.  Heads hold 27 bits.  The sampler reads the table alone when the blocks
+// leave more than kBlockMaxReads eighths of the samples to it (weights that the encoding does not
+// fit: then a sample would pay for both).
+constexpr uint32_t kBlockMinN = 1u << 22;
+constexpr uint32_t kBlockMaxN = 1u << 27;
+constexpr uint32_t kBlockMaxReads = 6;
 // The non-cooperative ITS sampler's bisection probes one implicit binary tree (node k, root
 // 1: the range left by the decisions spelled by the bits of k below its leading one).  The
 // build stores the tree's levels as blocks of three levels -- a node and its 6 descendants, 7

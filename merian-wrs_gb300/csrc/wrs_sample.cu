@@ -28,35 +28,78 @@ __device__ __forceinline__ float mix_rn(float x, float y, float a) {
     return __fadd_rn(__fmul_rn(x, __fsub_rn(1.0f, a)), __fmul_rn(y, a));
 }
 
-// The coin filter of a table: per bucket one byte q = floor(256 p) (255 for p >= 1, 0 for
-// p <= 0 or NaN), a lower bound of the bucket's keep threshold in both generator modes: a
-// coin below it (x1 < q * 2^24, or u < q / 256 for the shader's float coin) keeps the bucket
-// whatever its entry holds.  The sampler then reads the 8-byte entry only for the other
-// samples -- 1 - mean(q) / 256 of them: 0.42 for uniform weights, whose PSA buckets keep 58 %
-// of their draws -- while the filter (N bytes: 64 MB at N = 2^26) stays in L2 and the table
-// does not.
-// Every decision is the unfiltered one, so the samples are identical.
-__device__ __forceinline__ uint32_t coin_code(uint32_t pbits) {
-    const float p = __uint_as_float(pbits);
-    if (!(p > 0.0f)) return 0u;
-    if (p >= 1.0f) return 255u;
-    return static_cast<uint32_t>(__fmul_rn(p, 256.0f));  // exact product; truncation = floor
+// The eighth of [0, 1) a float p or coin u lies in: 0 for p <= 0 and NaN, 7 for values of 1 and
+// above (the product is exact, the conversion truncates and saturates).
+__device__ __forceinline__ uint32_t coin_cell_f(float p) {
+    return min(__float2uint_rz(__fmul_rn(p, 8.0f)), 7u);
 }
 
-// Samples [block * 1024 + 4t, +4) of one distribution (thread t of the CTA).  FILTER: coins is
-// the table's coin filter, read where `use` holds.
-template <uint32_t RNG, bool COOP, bool FILTER>
+// What a block says about a sample of bucket `self` whose coin lies in `cell`: the bucket itself,
+// its alias, or nothing (need: the entry must be read).
+struct BlockSays {
+    uint32_t r;
+    bool need;
+};
+__device__ __forceinline__ BlockSays block_says(const uint4& lo, const uint4& hi, uint32_t cell,
+                                                uint32_t self) {
+    const uint32_t b = self & 31u;
+    const uint32_t code = ((lo.x >> b) & 1u) | ((lo.y >> b) & 1u) << 1 | ((lo.z >> b) & 1u) << 2;
+    BlockSays s;
+    s.r = self;
+    s.need = cell == code;
+    if (cell > code) {
+        const uint32_t width = hi.x >> kAliasHeadBits;
+        const uint32_t up = lo.w >> b;  // bit 0: this bucket is heavy; then the buckets above it
+        if (up & 1u) {
+            // the distance to the next heavy bucket (0: beyond the block)
+            const uint32_t next = up & 0xfffffffeu;
+            s.r = self + (31u - static_cast<uint32_t>(__clz(static_cast<int>(next & (0u - next)))));
+            s.need = next == 0u || width == kAliasNone;
+        } else {
+            const uint32_t j = __popc(hi.y << (31u - b));  // switches up to this bucket
+            uint32_t d;
+            if (width == kAliasSteps) {
+                // the sum of the first j nibbles, and j
+                const uint64_t x = (static_cast<uint64_t>(hi.w) << 32 | hi.z) << (64u - 4u * j & 63u);
+                const uint32_t x0 = static_cast<uint32_t>(x), x1 = static_cast<uint32_t>(x >> 32);
+                d = __dp4a(x0 & 0x0f0f0f0fu, 0x01010101u, j);
+                d = __dp4a(x0 >> 4 & 0x0f0f0f0fu, 0x01010101u, d);
+                d = __dp4a(x1 & 0x0f0f0f0fu, 0x01010101u, d);
+                d = __dp4a(x1 >> 4 & 0x0f0f0f0fu, 0x01010101u, d);
+            } else {
+                const uint64_t off =
+                    (static_cast<uint64_t>(hi.w) << 32 | hi.z) >> ((j - 1u) * width & 63u);
+                d = static_cast<uint32_t>(off) & (0xffffffffu >> (32u - width & 31u));
+            }
+            s.r = (hi.x & kAliasHeadMask) + (j ? d : 0u);
+            s.need = width == kAliasNone;
+        }
+    }
+    return s;
+}
+
+// Samples [(256 block + t) PT, +PT) of one distribution (thread t of the CTA).  BLOCKS: blocks are
+// the table's alias blocks, consulted where `use` holds.
+//
+// By the table alone a sample is one random 8-byte read: from a table beyond L2 the device's rate of
+// random HBM accesses bounds it (50-70 G/s, whatever the bytes), from one in L2 the L1's one
+// wavefront per gathered sector (250 G/s).  Through the blocks (1 byte per bucket: 64 MB at n = 2^26,
+// mostly in L2) one 32-byte sector decides 86 % of uniform weights' samples and the bound is
+// instruction issue (72 % active, ~150 instructions per 32 samples; 22 % of the blocks still miss
+// L2 at 2^26): 2^28 samples, n = 2^26, uniform 2.76 -> 1.64 ms, log-normal(0, 2) 4.3 -> 1.73; 2 x 10^8
+// samples, n = 5 x 10^7, Zipf 3.3 -> 1.10 ms (against one byte of p per bucket, which decided only the
+// samples that their bucket keeps).
+template <uint32_t RNG, bool COOP, bool BLOCKS, int PT = kAliasPerThread>
 __device__ __forceinline__ void alias_block(const uint2* __restrict__ table,
-                                            const uint8_t* __restrict__ coins, bool use,
+                                            const AliasBlock* __restrict__ blocks, bool use,
                                             uint32_t n, uint64_t S, uint64_t seed,
                                             uint64_t offset, uint32_t coop,
                                             uint32_t* __restrict__ out, uint64_t block) {
     const uint64_t t = block * kSampleThreads + threadIdx.x;
-    const uint64_t s0 = t * kAliasPerThread;
+    const uint64_t s0 = t * PT;
     if (s0 >= S) return;
-    uint32_t r[kAliasPerThread];
-    uint64_t pol = 0;
-    if constexpr (FILTER) pol = l2_policy_evict_first();  // table entries: keep the filter in L2
+    uint32_t r[PT], ixs[PT];
+    uint32_t coin[PT];  // RNG_PHILOX: 32 bits; RNG_REF: the float coin's bits
     if constexpr (RNG == RNG_REF) {
         const uint32_t key = static_cast<uint32_t>(seed);
         const float fn = __uint2float_rn(n);
@@ -70,100 +113,89 @@ __device__ __forceinline__ void alias_block(const uint2* __restrict__ table,
             sx = __int2float_rn(ix - static_cast<int>(coop) / 2);
             sy = __int2float_rn(ix + static_cast<int>(coop) / 2);
         }
-        uint2 ent[kAliasPerThread];
-        int ixs[kAliasPerThread];
-        float uys[kAliasPerThread];
 #pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v) {
+        for (int v = 0; v < PT; ++v) {
             const uint32_t g = static_cast<uint32_t>(offset + s0 + v);
             const uint2 u = philox2x32_7(0u, g, key);
             const float ux = unit_ref(u.x);
-            uys[v] = unit_ref(u.y);
+            coin[v] = __float_as_uint(unit_ref(u.y));
             const float f = COOP ? mix_rn(sx, sy, ux) : __fmul_rn(fn, ux);
             int ix = __float2int_rz(f);
             ix = ix < 0 ? 0 : ix;
             ix = ix > static_cast<int>(n - 1u) ? static_cast<int>(n - 1u) : ix;
-            ixs[v] = ix;
-        }
-        if constexpr (FILTER) {
-            bool need[kAliasPerThread];
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v) need[v] = true;
-            if (use) {
-#pragma unroll
-                for (int v = 0; v < kAliasPerThread; ++v)
-                    need[v] = !(uys[v] <
-                                __fmul_rn(__uint2float_rn(__ldg(coins + ixs[v])), 0.00390625f));
-            }
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v)
-                ent[v] = need[v] ? ld_entry_policy(table + ixs[v], pol) : make_uint2(0u, 0u);
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v)
-                r[v] = need[v] && uys[v] >= __uint_as_float(ent[v].x) ? ent[v].y
-                                                                      : static_cast<uint32_t>(ixs[v]);
-        } else {
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v) ent[v] = ld_entry(table + ixs[v]);
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v)
-                r[v] = uys[v] >= __uint_as_float(ent[v].x) ? ent[v].y : static_cast<uint32_t>(ixs[v]);
+            ixs[v] = static_cast<uint32_t>(ix);
         }
     } else {
         uint2 ks[10];
         philox4x32_10_keys(seed, ks);
-        uint2 ent[kAliasPerThread];
-        uint32_t ixs[kAliasPerThread];
-        uint32_t coin[kAliasPerThread];
 #pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v) {
+        for (int v = 0; v < PT; ++v) {
             const uint64_t g = offset + s0 + v;
             const uint4 x = philox4x32_10(
                 make_uint4(static_cast<uint32_t>(g), static_cast<uint32_t>(g >> 32), 0u, 0u), ks);
             ixs[v] = __umulhi(x.x, n);
             coin[v] = x.y;
         }
-        bool need[kAliasPerThread];
-#pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v) need[v] = true;
-        if (FILTER && use) {
-#pragma unroll
-            for (int v = 0; v < kAliasPerThread; ++v)
-                need[v] = coin[v] >= (static_cast<uint32_t>(__ldg(coins + ixs[v])) << 24);
-        }
-#pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v) {
-            if constexpr (FILTER)
-                ent[v] = need[v] ? ld_entry_policy(table + ixs[v], pol) : make_uint2(0u, 0u);
-            else
-                ent[v] = ld_entry(table + ixs[v]);
-        }
-#pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v) {
-            const float p = __uint_as_float(ent[v].x);
-            const bool keep = !need[v] || p >= 1.0f ||
-                              coin[v] < __float2uint_ru(__fmul_rn(p, 4294967296.0f));
-            r[v] = keep ? ixs[v] : ent[v].y;
-        }
     }
-    if (s0 + kAliasPerThread <= S && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
-        __stcs(reinterpret_cast<uint4*>(out + s0), make_uint4(r[0], r[1], r[2], r[3]));
+    // whether the bucket keeps a sample, from its entry's p
+    auto keeps = [&](uint32_t c, uint32_t pbits) {
+        const float p = __uint_as_float(pbits);
+        if constexpr (RNG == RNG_REF) return !(__uint_as_float(c) >= p);
+        return p >= 1.0f || c < __float2uint_ru(__fmul_rn(p, 4294967296.0f));
+    };
+    bool blocked = false;
+    if constexpr (BLOCKS) blocked = use;
+    if (BLOCKS && blocked) {
+        const uint64_t once = l2_policy_evict_first();  // table entries: keep the blocks in L2
+        uint4 lo[PT], hi[PT];
+        bool need[PT];
+        uint2 ent[PT];
+#pragma unroll
+        for (int v = 0; v < PT; ++v)
+            ld_block(reinterpret_cast<const uint32_t*>(blocks + (ixs[v] >> 5)), lo[v], hi[v]);
+#pragma unroll
+        for (int v = 0; v < PT; ++v) {
+            const uint32_t cell =
+                RNG == RNG_REF ? coin_cell_f(__uint_as_float(coin[v])) : coin[v] >> 29;
+            const BlockSays s = block_says(lo[v], hi[v], cell, ixs[v]);
+            r[v] = s.r;
+            need[v] = s.need;
+            if (s.need) ent[v] = ld_entry_policy(table + ixs[v], once);
+        }
+#pragma unroll
+        for (int v = 0; v < PT; ++v)
+            if (need[v]) r[v] = keeps(coin[v], ent[v].x) ? ixs[v] : ent[v].y;
+    } else {
+        uint2 ent[PT];
+#pragma unroll
+        for (int v = 0; v < PT; ++v) ent[v] = ld_entry(table + ixs[v]);
+#pragma unroll
+        for (int v = 0; v < PT; ++v)
+            r[v] = keeps(coin[v], ent[v].x) ? ixs[v] : ent[v].y;
+    }
+    if (s0 + PT <= S && (reinterpret_cast<uintptr_t>(out) & (PT * 4u - 1u)) == 0) {
+        if constexpr (PT == 4)
+            __stcs(reinterpret_cast<uint4*>(out + s0), make_uint4(r[0], r[1], r[2], r[3]));
+        else if constexpr (PT == 2)
+            __stcs(reinterpret_cast<uint2*>(out + s0), make_uint2(r[0], r[1]));
+        else
+            __stcs(out + s0, r[0]);
     } else {
 #pragma unroll
-        for (int v = 0; v < kAliasPerThread; ++v)
+        for (int v = 0; v < PT; ++v)
             if (s0 + v < S) out[s0 + v] = r[v];
     }
 }
 
-template <uint32_t RNG, bool COOP, bool FILTER>
+template <uint32_t RNG, bool COOP, bool BLOCKS>
 __global__ __launch_bounds__(kSampleThreads) void k_alias_sample(
-    const uint2* __restrict__ table, const uint8_t* __restrict__ coins,
-    const unsigned long long* __restrict__ coin_sum, uint32_t n, uint64_t S, uint64_t seed,
+    const uint2* __restrict__ table, const AliasBlock* __restrict__ blocks,
+    const unsigned long long* __restrict__ reads, uint32_t n, uint64_t S, uint64_t seed,
     uint64_t offset, uint32_t coop, uint32_t* __restrict__ out) {
     pdl_entry();
     bool use = false;
-    if constexpr (FILTER) use = __ldg(coin_sum) >= kCoinMinMean * n;
-    alias_block<RNG, COOP, FILTER>(table, coins, use, n, S, seed, offset, coop, out, blockIdx.x);
+    if constexpr (BLOCKS) use = __ldg(reads) <= static_cast<unsigned long long>(kBlockMaxReads) * n;
+    alias_block<RNG, COOP, BLOCKS, BLOCKS ? kBlockPerThread : kAliasPerThread>(table, blocks, use, n, S, seed, offset, coop, out, blockIdx.x);
 }
 
 // All distributions of a batch in one launch: CTA b samples block b - sample0 of the
@@ -179,43 +211,111 @@ __global__ __launch_bounds__(kSampleThreads) void k_alias_sample_batch(BatchView
                                   D->out, blockIdx.x - D->sample0);
 }
 
-// The coin filter of table[0, n) (coin_code per entry, four entries per thread per step of a
-// grid-striding loop) and the sum of its codes, added into *coin_sum once per CTA.
-__global__ __launch_bounds__(kSampleThreads) void k_coin_filter(const uint2* __restrict__ table,
-                                                                uint32_t n,
-                                                                uint8_t* __restrict__ coins,
-                                                                unsigned long long* coin_sum) {
+// The alias blocks of table[0, n), one per thread, from its 32 entries (eight 32-byte loads, whole
+// sectors) and the partition's heavy bits.  0.105-0.111 ms at n = 2^26 (5.6 TB/s; HBM and the ALU
+// pipe about level).  One thread per block keeps the encoding serial and short, ~20 instructions per
+// entry; a lane per bucket (ballots and shuffles) would issue three times as many, and staging the
+// entries in shared memory for coalesced loads took 0.21 ms.  A block is encoded only where its aliases follow the rule that the
+// sampler decodes; where one does not (overlapping subproblems, distances that do not fit, a NaN)
+// the block keeps its codes and says so.  *reads receives 8 times the expected number of entry
+// reads by one sample of every bucket.
+__global__ __launch_bounds__(kBlockBuildThreads, 8) void k_alias_blocks(
+    const uint2* __restrict__ table, const uint32_t* __restrict__ classes, uint32_t n,
+    AliasBlock* __restrict__ blocks, unsigned long long* __restrict__ reads) {
     pdl_entry();
-    __shared__ unsigned long long s_sum[kSampleThreads / 32];
-    const uint64_t groups = (static_cast<uint64_t>(n) + 3u) / 4u;
-    const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kSampleThreads;
-    unsigned long long sum = 0;
-    for (uint64_t t = static_cast<uint64_t>(blockIdx.x) * kSampleThreads + threadIdx.x;
-         t < groups; t += stride) {
-        const uint64_t e0 = 4ull * t;
-        if (e0 + 4u <= n) {
-            const uint4 a = __ldcs(reinterpret_cast<const uint4*>(table + e0));
-            const uint4 b = __ldcs(reinterpret_cast<const uint4*>(table + e0 + 2u));
-            const uint32_t c0 = coin_code(a.x), c1 = coin_code(a.z), c2 = coin_code(b.x),
-                           c3 = coin_code(b.z);
-            reinterpret_cast<uint32_t*>(coins)[t] = c0 | c1 << 8 | c2 << 16 | c3 << 24;
-            sum += c0 + c1 + c2 + c3;
-        } else {
-            for (uint64_t e = e0; e < n; ++e) {
-                const uint32_t c = coin_code(table[e].x);
-                coins[e] = static_cast<uint8_t>(c);
-                sum += c;
+    __shared__ uint32_t s_sum[kBlockBuildThreads / 32];
+    const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
+    const uint64_t base64 =
+        (static_cast<uint64_t>(blockIdx.x) * kBlockBuildThreads + threadIdx.x) * 32u;
+    uint32_t sum = 0;
+    if (base64 < n) {
+        const uint32_t base = static_cast<uint32_t>(base64);
+        const uint32_t live = n - base >= 32u ? 0xffffffffu : (1u << (n - base)) - 1u;
+        const uint2* row = table + base;
+        const uint32_t cls = __ldg(classes + (base >> 5)) & live;
+        const uint32_t lights = ~cls & live;
+        const uint32_t head = lights ? __ldg(&row[__ffs(lights) - 1].y) : 0u;
+        uint32_t p0 = 0, p1 = 0, p2 = 0, sw = 0, odd = 0;
+        float nan = 0.0f;  // NaN once a p is (or is infinite)
+        uint32_t alias = head, heavy_alias = cls ? base + __ffs(cls) - 1u : 0u;
+        uint32_t step_max = 0, step_lo = 0, step_hi = 0;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            uint4 lo = make_uint4(0u, 0u, 0u, 0u), hi = lo;
+            if (live == 0xffffffffu) {
+                ld_block(reinterpret_cast<const uint32_t*>(row + 4 * q), lo, hi);
+            } else {
+                uint2 e[4];
+#pragma unroll
+                for (int c = 0; c < 4; ++c)
+                    e[c] = live >> (4 * q + c) & 1u ? __ldg(row + 4 * q + c) : make_uint2(0u, 0u);
+                lo = make_uint4(e[0].x, e[0].y, e[1].x, e[1].y);
+                hi = make_uint4(e[2].x, e[2].y, e[3].x, e[3].y);
+            }
+            const uint32_t px[4] = {lo.x, lo.z, hi.x, hi.z}, al[4] = {lo.y, lo.w, hi.y, hi.w};
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                const int i = 4 * q + c;
+                // p in [0, 1): floor(2 p), floor(4 p) and floor(8 p) in the low mantissa bits of
+                // 2^23 + k p rounded down (on the FMA pipe; the ALU pipe is the busier one)
+                const float p = __uint_as_float(px[c]);
+                const float q = fminf(__saturatef(p), 0x1.fffffep-1f);
+                p0 = __funnelshift_r(p0, __float_as_uint(__fmaf_rz(q, 8.0f, 8388608.0f)), 1);
+                p1 = __funnelshift_r(p1, __float_as_uint(__fmaf_rz(q, 4.0f, 8388608.0f)), 1);
+                p2 = __funnelshift_r(p2, __float_as_uint(__fmaf_rz(q, 2.0f, 8388608.0f)), 1);
+                nan = __fmaf_rn(p, 0.0f, nan);
+                const bool heavy = (cls & 1u << i) != 0u;
+                // the heavy bucket before does not alias this one
+                if (heavy && heavy_alias != base + i) odd |= 1u << i;
+                heavy_alias = heavy ? al[c] : heavy_alias;
+                // a light bucket with another alias than the light one before
+                const uint32_t step = al[c] - alias - 1u;  // (wraps where the aliases do not rise)
+                if (!heavy && step != 0xffffffffu) {
+                    sw |= 1u << i;
+                    step_lo = __funnelshift_r(step_lo, step_hi, 4);
+                    step_hi = __funnelshift_r(step_hi, step, 4);
+                    step_max = max(step_max, step);
+                }
+                alias = heavy ? alias : al[c];
             }
         }
+        const bool whole = live == 0xffffffffu;
+        sw &= live;
+        const uint32_t m = __popc(sw);
+        uint64_t off = 0;
+        uint32_t code = kAliasNone;
+        if (nan == 0.0f && odd == 0u && head <= kAliasHeadMask) {
+            if (whole && m <= 16u && step_max <= 15u) {
+                code = kAliasSteps;
+                off = m ? (static_cast<uint64_t>(step_hi) << 32 | step_lo) >> (64u - 4u * m) : 0u;
+            } else {
+                const uint32_t width = min(64u / max(m, 1u), 31u);  // bits per distance
+                uint32_t far = 0, at = 0;
+                for (uint32_t rest = sw; rest; rest &= rest - 1u, at += width) {
+                    const uint32_t d = __ldg(&row[__ffs(rest) - 1].y) - head;
+                    off |= static_cast<uint64_t>(d) << at;
+                    far |= d;
+                }
+                if (width > kAliasSteps && far >> width == 0u) code = width;
+            }
+        }
+        uint4* dst = reinterpret_cast<uint4*>(blocks + (base >> 5));
+        dst[0] = make_uint4(p0, p1, p2, cls);
+        dst[1] = make_uint4((head & kAliasHeadMask) | code << kAliasHeadBits, sw,
+                            static_cast<uint32_t>(off), static_cast<uint32_t>(off >> 32));
+        // entry reads, in eighths of a sample per bucket: coins in the bucket's own cell, or all
+        // above it
+        sum = __popc(live);
+        if (code == kAliasNone)
+            sum = 8u * sum - __popc(p0 & live) - 2u * __popc(p1 & live) - 4u * __popc(p2 & live);
     }
-#pragma unroll
-    for (int m = 16; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-    if ((threadIdx.x & 31) == 0) s_sum[threadIdx.x >> 5] = sum;
+    sum = __reduce_add_sync(0xffffffffu, sum);
+    if (lane == 0) s_sum[warp] = sum;
     __syncthreads();
     if (threadIdx.x == 0) {
-        unsigned long long tot = 0;
-        for (int w = 0; w < kSampleThreads / 32; ++w) tot += s_sum[w];
-        atomicAdd(coin_sum, tot);
+        uint32_t tot = 0;
+        for (int w = 0; w < kBlockBuildThreads / 32; ++w) tot += s_sum[w];
+        atomicAdd(reads, static_cast<unsigned long long>(tot));
     }
 }
 
@@ -1200,40 +1300,41 @@ cudaError_t launch_cutpoint_sample(cudaStream_t st, uint32_t rng, const float* c
 }
 
 cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, const uint2* table,
-                                const uint8_t* coins, const unsigned long long* coin_sum,
+                                const AliasBlock* blocks, const unsigned long long* reads,
                                 uint32_t n, uint64_t S, uint64_t seed, uint64_t offset,
                                 uint32_t* out) {
-    const uint64_t threads = (S + kAliasPerThread - 1) / kAliasPerThread;
-    const uint64_t blocks = (threads + kSampleThreads - 1) / kSampleThreads;
-    if (blocks == 0) return cudaSuccess;
-    if (blocks > 0x7fffffffull) return cudaErrorInvalidValue;
-    const dim3 grid(static_cast<unsigned>(blocks));
-    const uint8_t* c = coop || !coin_sum ? nullptr : coins;  // cooperative: the table alone
+    const bool b = blocks && reads && !coop;  // cooperative: the table alone
+    const uint64_t per = b ? kBlockPerThread : kAliasPerThread;
+    const uint64_t threads = (S + per - 1) / per;
+    const uint64_t ctas = (threads + kSampleThreads - 1) / kSampleThreads;
+    if (ctas == 0) return cudaSuccess;
+    if (ctas > 0x7fffffffull) return cudaErrorInvalidValue;
+    const dim3 grid(static_cast<unsigned>(ctas));
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed, offset, coop, out);
+    };
     if (rng == RNG_REF) {
         if (coop)
-            launch_pdl(k_alias_sample<RNG_REF, true, false>, grid, kSampleThreads, 0, st, table, c, coin_sum, n, S, seed, offset, coop, out);
-        else if (c)
-            launch_pdl(k_alias_sample<RNG_REF, false, true>, grid, kSampleThreads, 0, st, table, c, coin_sum, n, S, seed, offset, coop, out);
+            go(k_alias_sample<RNG_REF, true, false>);
+        else if (b)
+            go(k_alias_sample<RNG_REF, false, true>);
         else
-            launch_pdl(k_alias_sample<RNG_REF, false, false>, grid, kSampleThreads, 0, st, table, c, coin_sum, n, S, seed, offset, coop, out);
-    } else if (c) {
-        launch_pdl(k_alias_sample<RNG_PHILOX, false, true>, grid, kSampleThreads, 0, st, table, c, coin_sum, n, S, seed, offset, coop, out);
+            go(k_alias_sample<RNG_REF, false, false>);
+    } else if (b) {
+        go(k_alias_sample<RNG_PHILOX, false, true>);
     } else {
-        launch_pdl(k_alias_sample<RNG_PHILOX, false, false>, grid, kSampleThreads, 0, st, table, c, coin_sum, n, S, seed, offset, coop, out);
+        go(k_alias_sample<RNG_PHILOX, false, false>);
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_coin_filter(cudaStream_t st, const uint2* table, uint32_t n, uint8_t* coins,
-                               unsigned long long* coin_sum) {
-    const uint64_t groups = (static_cast<uint64_t>(n) + 3u) / 4u;
-    const uint64_t blocks = (groups + kSampleThreads - 1) / kSampleThreads;
-    if (blocks == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(coin_sum, 0, sizeof(*coin_sum), st);
+cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint32_t* classes,
+                                uint32_t n, AliasBlock* blocks, unsigned long long* reads) {
+    cudaError_t e = cudaMemsetAsync(reads, 0, sizeof(*reads), st);
     if (e != cudaSuccess) return e;
-    // a few CTAs per SM, striding over the table: one atomic per CTA
-    const unsigned grid = static_cast<unsigned>(blocks < 8u * 152u ? blocks : 8u * 152u);
-    launch_pdl(k_coin_filter, grid, kSampleThreads, 0, st, table, n, coins, coin_sum);
+    constexpr uint32_t span = kBlockBuildThreads * 32u;  // entries per CTA
+    launch_pdl(k_alias_blocks, static_cast<unsigned>((static_cast<uint64_t>(n) + span - 1) / span),
+               kBlockBuildThreads, 0, st, table, classes, n, blocks, reads);
     return cudaGetLastError();
 }
 
