@@ -139,14 +139,15 @@ def launches_per_step(n: int) -> int:
     return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 27))
 
 
-def profiled_traffic(l2_fetch: int) -> float | None:
-    """DRAM bytes of one headline alias-sampling launch (through the tables' alias blocks, the
-    mean over the three distributions' launches) at the given L2 fetch granularity, from the
-    committed ncu summary (a line `dram_bytes_per_launch_blocks[l2=B]: X` per captured
-    granularity), if it holds that granularity."""
+def profiled_traffic(l2_fetch: int, kernel: str = "coin_filter") -> float | None:
+    """DRAM bytes of one headline alias-sampling launch (the mean over the three distributions'
+    launches) at the given L2 fetch granularity, from the committed ncu summary (a line
+    `dram_bytes_per_launch_<kernel>[l2=B]: X` per captured granularity), if it holds that
+    granularity.  kernel: "blocks", the sampler through the alias blocks, or "coin_filter", the
+    sampler before them."""
     if not os.path.exists(PROFILE_TRAFFIC):
         return None
-    key = f"dram_bytes_per_launch_blocks[l2={l2_fetch}]:"
+    key = f"dram_bytes_per_launch_{kernel}[l2={l2_fetch}]:"
     for line in open(PROFILE_TRAFFIC):
         if line.strip().startswith(key):
             return float(line.split(":", 1)[1].split()[0])
@@ -548,7 +549,7 @@ def main() -> None:
     pk = peaks()
     samp_s = statistics.mean(sample_ms) / 1e3
     achieved = 12.0 * s / samp_s / 1e9
-    traffic = profiled_traffic(tune["l2_fetch"])
+    traffic = profiled_traffic(tune["l2_fetch"], "blocks")
     gather_rate = random_gather_rate(W, internals, n, s, stream)
     roofline = {"bound": "hbm", "achieved": achieved, "peak": pk["hbm_gbs"], "unit": "GB/s",
                 "frac": achieved / pk["hbm_gbs"], "traffic": traffic,
