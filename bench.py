@@ -134,9 +134,9 @@ def peaks() -> dict:
 def launches_per_step(n: int) -> int:
     """The library's kernel launches in one headline step (wrs_build + wrs_sample): total mass,
     partition, the split descent (split-pack grids of >= 512 CTAs of 479 subproblems), the
-    split-pack, the alias blocks (2^22 < N <= 2^27) and the sampler."""
+    split-pack, the alias blocks (2^22 < N <= 2^26) and the sampler."""
     blocks = -(-(n // SPLIT_SIZE) // 479)
-    return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 27))
+    return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 26))
 
 
 def profiled_traffic(l2_fetch: int, kernel: str = "coin_filter") -> float | None:

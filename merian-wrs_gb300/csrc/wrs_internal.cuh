@@ -203,12 +203,12 @@ cudaError_t launch_split_pack(cudaStream_t st, bool r64, bool full_light, const 
 struct alignas(32) AliasBlock {
     uint32_t code[3];
     uint32_t cls;
-    uint32_t head;  // alias (27 bits) | width << 27
+    uint32_t head;  // alias (26 bits) | width << 26
     uint32_t sw;
     uint32_t off[2];
 };
 static_assert(sizeof(AliasBlock) == 32, "one alias block is one 32-byte sector");
-constexpr uint32_t kAliasHeadBits = 27;
+constexpr uint32_t kAliasHeadBits = 26;
 constexpr uint32_t kAliasHeadMask = (1u << kAliasHeadBits) - 1u;
 // widths that say something else: the aliases are not encoded; `off` holds steps
 constexpr uint32_t kAliasNone = 0, kAliasSteps = 1;
@@ -231,12 +231,11 @@ cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint3
 // costs its 32-byte sector and the decoding (190 G samples/s while the blocks stay in L2); by the
 // table alone it costs its 8-byte entry, 250 G/s from L2 and 50 G/s from HBM.  2^26 samples of
 // uniform weights, us, by the table / through the blocks: n = 4.0 M 274 / 352, 6.0 M 423 / 353,
-// 8.0 M 549 / 353, 12 M 749 / 355; 2^28 samples: n = 2^26 5300 / 1640, 2^27 (blocks of 128 MB, half of
-// them in L2) 5508 / 3064.  Heads hold 27 bits.  The sampler reads the table alone when the blocks
-// leave more than kBlockMaxReads eighths of the samples to it (weights that the encoding does not
-// fit: then a sample would pay for both).
+// 8.0 M 549 / 353, 12 M 749 / 355; 2^28 samples: n = 2^26 5300 / 1640.  Beyond 2^26 the blocks no longer
+// fit L2.  The sampler reads the table alone when the blocks leave more than kBlockMaxReads eighths
+// of the samples to it (weights that the encoding does not fit: then a sample would pay for both).
 constexpr uint32_t kBlockMinN = 1u << 22;
-constexpr uint32_t kBlockMaxN = 1u << 27;
+constexpr uint32_t kBlockMaxN = 1u << 26;
 constexpr uint32_t kBlockMaxReads = 6;
 // The non-cooperative ITS sampler's bisection probes one implicit binary tree (node k, root
 // 1: the range left by the decisions spelled by the bits of k below its leading one).  The
