@@ -134,13 +134,14 @@ typedef struct wrs_config {
                                         light bucket extra mass; 0 = reference behaviour */
     uint32_t guiding_entry_size;     /* Cutpoint: CutpointConfig::guidingEntrySize, weights per
                                         guiding-table entry (table size ceil(N / this));
-                                        default 32.  ITS with coop 0: the CMF is cut into as
-                                        many equal-mass cells, each stored as a 32-byte block
-                                        (its index range and 6 CMF values), and each sample
-                                        reads the block of its cell instead of bisecting the
-                                        whole CMF, with the same index: the compensated CMF is
-                                        exactly non-decreasing; on an FP32 CMF the build marks
-                                        the cells whose targets can meet a decrease of the CMF,
+                                        default 32.  ITS with coop 0: the CMF is cut into
+                                        equal-mass cells of about so many weights (twice to
+                                        four times as many on the compensated CMF), each stored
+                                        as a 32-byte block, and each sample reads the block of
+                                        its cell instead of bisecting the whole CMF, with the
+                                        same index: the compensated CMF is exactly
+                                        non-decreasing; on an FP32 CMF the build marks the
+                                        cells whose targets can meet a decrease of the CMF,
                                         and those samples bisect.  Default 4 for ITS; 0 = no
                                         cells (the bisection through the stored probe tree) */
     uint32_t split_pack_mode;        /* wrs_split_pack_mode: PSAConfig's splitPack alternative;

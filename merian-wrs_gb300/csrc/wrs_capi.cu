@@ -50,10 +50,11 @@ struct wrs_buffers {
     SplitRecord* records = nullptr;  // serial split-pack
     float* cmf = nullptr;
     uint32_t* guide = nullptr;
-    ItsCell* cells = nullptr;
+    ItsCell* cells = nullptr;    // ITS: the FP32 CMF's cells, or the compensated CMF's grid
     TreeBlock* tree = nullptr;   // ITS bisection: the probe tree's stored block levels
     uint32_t tree_n = 0;         // the n the last build stored them for (0: none)
-    uint32_t cells_n = 0;        // the n the last build wrote the ITS cell blocks for (0: none)
+    uint32_t cells_n = 0;        // the n the last build wrote them for (0: none)
+    bool cells_grid = false;     // the last build wrote the grid
     AliasBlock* blocks = nullptr;  // alias: the table's alias blocks (kBlockMinN < n)
     uint32_t* classes = nullptr;   // the partition's heavy bits, for the blocks
     uint32_t blocks_n = 0;         // the n the last build wrote the alias blocks for (0: none)
@@ -146,7 +147,7 @@ Layout layout_for(const wrs_config& cfg, uint32_t max_n) {
         if (!its)
             L.guide = take(sizeof(uint32_t) * G);
         else if (G)
-            L.cells = take(sizeof(ItsCell) * G);
+            L.cells = take(sizeof(ItsCell) * G);  // (the grid has fewer cells, of the same size)
         if (G && (its || cfg.scan_precision != WRS_SCAN_FP32))
             L.coarse = take(sizeof(uint32_t) * (coarse_entries(G) + group_entries(G)));
         // ITS bisecting the whole CMF (FP32, or no cells): the probe tree's deeper levels
@@ -550,14 +551,20 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
                           : launch_cutpoint_guide(st, b->cmf, n, G, b->guide),
                      "guiding table");
         else if (its_guided(h)) {
-            // an FP32 CMF need not be monotone: mark the cells the search cannot serve
             b->cells_n = 0;
-            WRS_CUDA(launch_its_cells(st, b->cmf, n, G, b->coarse, b->cells, !comp), "ITS cells");
-            if (!comp)
+            b->cells_grid = comp;
+            if (comp) {
+                WRS_CUDA(launch_its_grids(st, b->cmf, n, its_grids(n, h->cfg.guiding_entry_size),
+                                          b->coarse, reinterpret_cast<ItsGrid*>(b->cells)),
+                         "ITS grid");
+            } else {
+                // an FP32 CMF need not be monotone: mark the cells the search cannot serve
+                WRS_CUDA(launch_its_cells(st, b->cmf, n, G, b->coarse, b->cells), "ITS cells");
                 WRS_CUDA(launch_its_marks(st, b->cmf, n, G, b->cells,
                                           reinterpret_cast<float*>(b->tile_scratch),
                                           b->tile_scratch + 2u * b->cap_tiles),
                          "ITS cell marks");
+            }
             b->cells_n = n;
         }
         b->tree_n = 0;
@@ -623,14 +630,22 @@ wrs_status wrs_sample_at(const wrs_handle* h, void* stream, const wrs_buffers* b
         return fail(WRS_ERR_INVALID_ARG, "buffers were created for another method");
     if ((st = check_tables(h, b)) != WRS_OK) return st;
     if (h->cfg.method == WRS_METHOD_ITS) {
-        if (its_guided(h) && s && b->cells_n == n) {
-            // the cell-block search returns the bisection's index: for every target on the
-            // compensated (non-decreasing) CMF, for the unmarked cells' targets on an FP32 one;
-            // the marked cells bisect, through the stored probe tree when the build made it.
-            // Cells written for another n (or none yet) are not read: the bisections below
-            // give the same samples
+        if (its_guided(h) && s && b->cells_n == n && b->cells_grid == compensated(h)) {
+            // the grid's search returns the bisection's index for every target on the
+            // compensated (non-decreasing) CMF, the cells' for the unmarked cells' targets on an
+            // FP32 one; the marked cells bisect, through the stored probe tree when the build
+            // made it.  Cells or a grid written for another n (or none yet) are not read: the
+            // bisections below give the same samples
             if (!samples) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
-            const bool tree = !compensated(h) && b->tree && b->tree_n == n;
+            if (compensated(h)) {
+                WRS_CUDA(launch_its_sample_grids(as_stream(stream), h->cfg.rng, b->cmf, n,
+                                                 reinterpret_cast<const ItsGrid*>(b->cells),
+                                                 its_grids(n, h->cfg.guiding_entry_size), s, seed,
+                                                 offset, samples),
+                         "its sample");
+                return WRS_OK;
+            }
+            const bool tree = b->tree && b->tree_n == n;
             WRS_CUDA(launch_its_sample_cells(as_stream(stream), h->cfg.rng, b->cmf, n, b->cells,
                                              guide_entries(n, h->cfg.guiding_entry_size), s,
                                              seed, offset, samples, tree ? b->tree : nullptr,

@@ -299,9 +299,9 @@ __host__ __device__ inline uint32_t coarse_entries(uint32_t G) {
 __host__ __device__ inline uint32_t group_entries(uint32_t G) { return (G + 31u) / 32u + 1u; }
 cudaError_t launch_guide_monotone(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                   uint32_t* coarse, uint32_t* guide);
-// ITS on a non-decreasing CMF through cell blocks: cell k of G equal-mass cells (the Cutpoint
-// guiding table's) = its candidate range [x, y] and the CMF at the last index of each of the
-// range's kCellParts parts of d = ceil((y - x + 1) / kCellParts) indices; one 32-byte sector
+// ITS on the FP32 CMF through cells: cell k of G equal-mass cells (the Cutpoint guiding table's) =
+// its candidate range [x, y] and the CMF at the last index of each of the range's kCellParts parts
+// of d = ceil((y - x + 1) / kCellParts) indices; one 32-byte sector
 constexpr int kCellParts = 6;
 struct alignas(32) ItsCell {
     uint32_t x, y;
@@ -309,13 +309,42 @@ struct alignas(32) ItsCell {
 };
 static_assert(sizeof(ItsCell) == 32, "one cell block is one 32-byte sector");
 cudaError_t launch_its_cells(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsCell* cells, bool check = false);
+                             uint32_t* coarse, ItsCell* cells);
 cudaError_t launch_its_sample_cells(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
                                     const ItsCell* cells, uint32_t G, uint64_t S, uint64_t seed,
-                                    uint64_t offset, uint32_t* out,
-                                    const TreeBlock* blocks = nullptr, uint32_t L = 0);
+                                    uint64_t offset, uint32_t* out, const TreeBlock* blocks,
+                                    uint32_t L);
+// ITS on the compensated (exactly non-decreasing) CMF: F(v) = floor(v * 2^s) cuts the CMF's values
+// into cells of 128 steps, the power 2^s such that at most its_grids(n, entry) cells hold them
+// (its_scale).  Cell k = F >> 7 is one 32-byte sector: the first index x with F(cmf[x]) >= 128 k and,
+// for up to kGridSlots parts of 2^e items from x on, the step (7 bits) of each part's last item.
+// The product is exact and F monotone, so an item of a lower step than a target's is below it and
+// one of a higher step is not, and of equal steps >= 2^23 (where values are whole steps) neither is
+// below the other: a target is settled by its cell alone unless it shares a step with an item
+// below 2^23, or the cell's parts hold several items.
+constexpr int kGridSlots = 27;
+constexpr uint32_t kGridSteps = 128;
+struct alignas(32) ItsGrid {
+    uint32_t x;
+    uint32_t q[7];  // bytes: kGridSlots times 128 + step (255 past the cell's items), then e
+};
+static_assert(sizeof(ItsGrid) == 32, "one grid cell is one 32-byte sector");
+// cells for n weights: 2 to 4 times `entry` items each (the power of two leaves a factor of two),
+// and no more than FP32 values tell apart.  Against 3 to 6 times, with entry 4, build / 2^26 samples,
+// us: log-normal n = 2^24 162 / 400 and 147 / 478, n = 10^6 45 / 429 and 45 / 520 (fewer items in a
+// target's own step, fewer cells with more items than parts); uniform n = 2^24 161 / 343, 145 / 344
+__host__ __device__ inline uint32_t its_grids(uint32_t n, uint32_t entry) {
+    const uint64_t per = 2ull * entry;
+    const uint64_t g = (n + per - 1) / per;
+    return static_cast<uint32_t>(g < (1u << 24) ? g : (1u << 24));
+}
+cudaError_t launch_its_grids(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
+                             uint32_t* coarse, ItsGrid* grids);
+cudaError_t launch_its_sample_grids(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
+                                    const ItsGrid* grids, uint32_t G, uint64_t S, uint64_t seed,
+                                    uint64_t offset, uint32_t* out);
 // FP32 CMF: marks the cells whose targets can meet a decrease of the CMF (bit 31 of y), after
-// launch_its_cells with check (which marks the cells whose start is not below c_k);
+// launch_its_cells (which marks the cells whose start is not below c_k);
 // tile_scratch: 2 * tiles_for(n) floats; bad: a device word (set when every cell is marked)
 cudaError_t launch_its_marks(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                              ItsCell* cells, float* tile_scratch, uint32_t* bad);

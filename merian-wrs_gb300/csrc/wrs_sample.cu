@@ -691,11 +691,13 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_tree(const float*
     }
 }
 
-// ---- ITS on an exactly non-decreasing CMF: cell blocks ----------------------------------
+// ---- ITS through cells ---------------------------------------------------------------------
 //
 // On a non-decreasing CMF every lower-bound search returns the same index, so the search can
-// start anywhere that brackets the answer (the compensated scan's CMF is non-decreasing by
-// construction).  The CMF's range is cut into G = ceil(N / entry) cells of equal mass, the
+// start anywhere that brackets the answer.  The compensated scan's CMF is non-decreasing by
+// construction: its grid is below (ItsGrid).  The FP32 scan's CMF nearly is: its cells (ItsCell)
+// are read where a target cannot meet a decrease (below), as follows.
+// The CMF's range is cut into G = ceil(N / entry) cells of equal mass, the
 // Cutpoint guiding table's: cell k starts at x_k = lower bound of c_k = fl(fl(total / G) * k),
 // and a target T with c_k < T <= c_{k+1} has its lower bound in [x_k, y_k], y_k = x_{k+1}
 // (N - 1 for the last cell).  Cell k is stored as one 32-byte block (ItsCell): x_k, y_k and,
@@ -718,10 +720,37 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_tree(const float*
 // pass and each start is the bracket's start plus the number of values below its threshold,
 // found by a bisection over the values held in the warp's registers (shuffles, no dependent
 // loads); wider brackets are bisected in memory.
-__device__ __forceinline__ float cell_step(const float* __restrict__ cmf, uint32_t n, uint32_t G) {
-    return __fdiv_rn(__ldg(cmf + n - 1u), __uint2float_rn(G));
+//
+// GRID: the thresholds of the compensated ITS grid, c_k = 128 k 2^-s, exact for k <= 2^24.
+// 2^s for a CMF of the given total and at most G cells: floor(total * 2^s) < 128 G (and within a
+// factor of two of it, but for totals below 2^-96, whose power is capped)
+__device__ __forceinline__ int its_shift(float total, uint32_t G) {
+    const uint32_t e = __float_as_uint(total) >> 23;
+    if (e == 0u) return 127;           // zero or denormal: F < 2^(127 - 126) steps
+    if (e >= 255u) return 7;           // not finite (or negative): results are meaningless
+    const int E = 31 - __clz(static_cast<int>(G));
+    // total = m 2^(e - 127), 1 <= m < 2: total * 2^s / 128 = m 2^E or half of it
+    const float m = __uint_as_float((__float_as_uint(total) & 0x7fffffu) | 0x3f800000u);
+    const bool half = __fmul_rn(m, __uint_as_float(static_cast<uint32_t>(E + 127) << 23)) >=
+                      __uint2float_rn(G);
+    return min(E - (static_cast<int>(e) - 127) - (half ? 1 : 0) + 7, 127);
+}
+__device__ __forceinline__ float pow2f(int e) {
+    return __uint_as_float(static_cast<uint32_t>(e + 127) << 23);
 }
 
+template <bool GRID>
+__device__ __forceinline__ float cell_step(const float* __restrict__ cmf, uint32_t n, uint32_t G) {
+    const float total = __ldg(cmf + n - 1u);
+    if constexpr (GRID) return pow2f(7 - its_shift(total, G));  // (unused for G = 1)
+    return __fdiv_rn(total, __uint2float_rn(G));
+}
+// threshold c_k of cell k
+__device__ __forceinline__ float cell_at(float step, uint32_t k) {
+    return k ? __fmul_rn(step, __uint2float_rn(k)) : 0.0f;
+}
+
+template <bool GRID>
 __global__ __launch_bounds__(kSampleThreads) void k_cell_coarse(const float* __restrict__ cmf,
                                                                 uint32_t n, uint32_t G,
                                                                 uint32_t* __restrict__ coarse) {
@@ -730,21 +759,22 @@ __global__ __launch_bounds__(kSampleThreads) void k_cell_coarse(const float* __r
     if (j >= coarse_entries(G)) return;
     const uint64_t k = static_cast<uint64_t>(j) * kCoarseStride;
     coarse[j] = k < G ? bisect(cmf, 0, n - 1u,
-                               __fmul_rn(cell_step(cmf, n, G), __uint2float_rn(static_cast<uint32_t>(k))))
+                               cell_at(cell_step<GRID>(cmf, n, G), static_cast<uint32_t>(k)))
                       : n - 1u;
 }
 
+template <bool GRID>
 __device__ __forceinline__ uint32_t cell_start(const float* __restrict__ cmf, uint32_t n,
                                                uint32_t G, const uint32_t* __restrict__ coarse,
                                                uint32_t k) {
     const uint32_t j = k / kCoarseStride;
     const uint32_t lo = __ldg(coarse + j);
     if (k % kCoarseStride == 0u) return lo;
-    return bisect(cmf, lo, __ldg(coarse + j + 1u),
-                  __fmul_rn(cell_step(cmf, n, G), __uint2float_rn(k)));
+    return bisect(cmf, lo, __ldg(coarse + j + 1u), cell_at(cell_step<GRID>(cmf, n, G), k));
 }
 
 // group[g] = x_{32 g} (N - 1 past the last cell), g <= ceil(G / 32)
+template <bool GRID>
 __global__ __launch_bounds__(kSampleThreads) void k_cell_groups(const float* __restrict__ cmf,
                                                                 uint32_t n, uint32_t G,
                                                                 const uint32_t* __restrict__ coarse,
@@ -753,11 +783,12 @@ __global__ __launch_bounds__(kSampleThreads) void k_cell_groups(const float* __r
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= group_entries(G)) return;
     const uint64_t k = static_cast<uint64_t>(g) * 32u;
-    group[g] = k < G ? cell_start(cmf, n, G, coarse, static_cast<uint32_t>(k)) : n - 1u;
+    group[g] = k < G ? cell_start<GRID>(cmf, n, G, coarse, static_cast<uint32_t>(k)) : n - 1u;
 }
 
 // The start of cell k = 32 g + lane (all lanes of the warp call it; k >= G returns N - 1), and
 // the end of the group's bracket in hi.
+template <bool GRID>
 __device__ __forceinline__ uint32_t cell_start_warp(const float* __restrict__ cmf, uint32_t n,
                                                     uint32_t G, const uint32_t* __restrict__ group,
                                                     uint32_t g, uint32_t& hi) {
@@ -765,8 +796,7 @@ __device__ __forceinline__ uint32_t cell_start_warp(const float* __restrict__ cm
     const uint32_t lo = __ldg(group + g);
     hi = __ldg(group + g + 1u);
     const uint32_t k = g * 32u + lane;
-    const float t = k < G ? __fmul_rn(cell_step(cmf, n, G), __uint2float_rn(k))
-                          : __int_as_float(0x7f800000);
+    const float t = k < G ? cell_at(cell_step<GRID>(cmf, n, G), k) : __int_as_float(0x7f800000);
     uint32_t x;
     if (hi >= lo && hi - lo < 128u) {
         // values lo .. lo + 127, 4 consecutive per lane (past hi or N: +inf, never below t)
@@ -810,9 +840,8 @@ __device__ __forceinline__ uint32_t cell_part(uint32_t x, uint32_t y) {
     return (y - x + kCellParts) / kCellParts;  // ceil((y - x + 1) / kCellParts)
 }
 
-// CHECK (an FP32 CMF, which need not be monotone): a cell whose start x > 0 does not have
-// cmf[x - 1] < c_k is marked for the bisection as it is written
-template <bool CHECK>
+// the FP32 CMF need not be monotone: a cell whose start x > 0 does not have cmf[x - 1] < c_k is
+// marked for the bisection as it is written
 __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __restrict__ cmf,
                                                               uint32_t n, uint32_t G,
                                                               const uint32_t* __restrict__ group,
@@ -821,7 +850,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __res
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
-    const uint32_t x = cell_start_warp(cmf, n, G, group, g, hi);
+    const uint32_t x = cell_start_warp<false>(cmf, n, G, group, g, hi);
     const uint32_t k = g * 32u + (threadIdx.x & 31u);
     // the end of a cell is the next cell's start: the next lane's, or the next group's
     uint32_t y = __shfl_down_sync(0xffffffffu, x, 1);
@@ -834,14 +863,171 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __res
     for (int j = 0; j < kCellParts; ++j)
         v[j] = __ldg(cmf + min(x + (j + 1) * d - 1u, y));
     uint32_t ym = y;
-    if (CHECK && x > 0u) {
-        const float ck = __fmul_rn(cell_step(cmf, n, G), __uint2float_rn(k));
+    if (x > 0u) {
+        const float ck = cell_at(cell_step<false>(cmf, n, G), k);
         if (!(x <= n - 1u && __ldg(cmf + x - 1u) < ck)) ym |= kCellUnsafe;
     }
     uint4* dst = reinterpret_cast<uint4*>(cells + k);
     dst[0] = make_uint4(x, ym, __float_as_uint(v[0]), __float_as_uint(v[1]));
     dst[1] = make_uint4(__float_as_uint(v[2]), __float_as_uint(v[3]), __float_as_uint(v[4]),
                         __float_as_uint(v[5]));
+}
+
+// ---- the grid of the compensated CMF ------------------------------------------------------
+
+__device__ __forceinline__ uint32_t grid_f(float v, float scale) {
+    return __float2uint_rz(__fmul_rn(v, scale));  // (exact product; NaN and negative values: 0)
+}
+
+// One cell per lane, a warp per 32 (cell_start_warp finds their starts): the steps of its parts'
+// last items.  0.051 ms at n = 2^24 (2^21 cells, 64 MB written, the CMF read once from HBM: 2.6
+// TB/s), issue-bound: 27 loads and conversions a cell.
+__global__ __launch_bounds__(kSampleThreads) void k_its_grids(const float* __restrict__ cmf,
+                                                              uint32_t n, uint32_t G,
+                                                              const uint32_t* __restrict__ group,
+                                                              ItsGrid* __restrict__ grids) {
+    pdl_entry();
+    const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
+    if (g * 32u >= G) return;
+    uint32_t hi;
+    const uint32_t x = cell_start_warp<true>(cmf, n, G, group, g, hi);
+    const uint32_t k = g * 32u + (threadIdx.x & 31u);
+    uint32_t y = __shfl_down_sync(0xffffffffu, x, 1);
+    if ((threadIdx.x & 31u) == 31u) y = hi;
+    if (k >= G) return;
+    if (k + 1u >= G) y = n - 1u;
+    const uint32_t m = y > x ? y - x : 0u;  // items of the cell (y itself is the next cell's first)
+    uint32_t e = 0;
+    while ((static_cast<uint64_t>(kGridSlots) << e) < m) ++e;
+    const uint32_t parts = m >> e;  // whole parts (the rest is below y, the next cell's first)
+    const float scale = pow2f(its_shift(__ldg(cmf + n - 1u), G));
+    uint32_t w[8];
+    w[0] = x;
+#pragma unroll
+    for (int c = 0; c < 7; ++c) {
+        uint32_t f[4];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t j = 4u * c + i;
+            f[i] = 127u;
+            if (j < kGridSlots && j < parts)
+                f[i] = grid_f(__ldg(cmf + x + ((j + 1u) << e) - 1u), scale) & 127u;
+        }
+        w[1 + c] = 0x80808080u | f[0] | f[1] << 8 | f[2] << 16 | f[3] << 24;
+    }
+    w[7] = (w[7] & 0xffffffu) | e << 24;
+    uint4* dst = reinterpret_cast<uint4*>(grids + k);
+    dst[0] = make_uint4(w[0], w[1], w[2], w[3]);
+    dst[1] = make_uint4(w[4], w[5], w[6], w[7]);
+}
+
+// The smallest float that is not below T = (2x + 1) * total * 2^-33: "T > c" for a float c is
+// "its_target > c".
+__device__ __forceinline__ float its_target(uint32_t x, float total) {
+    const uint32_t e = __float_as_uint(total) >> 23;
+    if (e >= 67u && e < 255u) {  // total >= 2^-60: every power below is normal
+        // total = mt * 2^(e - 150): the 57-bit product rounded up to 24 bits, then scaled exactly
+        const uint32_t mt = (__float_as_uint(total) & 0x7fffffu) | 0x800000u;
+        const uint64_t P = (static_cast<uint64_t>(x) * mt << 1) + mt;
+        return __fmul_rn(__ull2float_ru(P), pow2f(static_cast<int>(e) - 150 - 33));
+    }
+    float t_hi;
+    int t_sgn;
+    exact_target(x, total, t_hi, t_sgn);
+    return t_sgn > 0 ? __uint_as_float(__float_as_uint(t_hi) + 1u) : t_hi;
+}
+
+// Samples per thread: two blocks of 8 words leave room for a full SM of warps.
+constexpr int kGridPerThread = 2;
+
+// One 32-byte sector of the grid (2 to 4 bytes per weight at entry 4) settles a sample, with no
+// division and no search for its cell.  n = 2^24, 2^26 samples: log-normal 0.97 -> 0.40 ms, uniform
+// 0.91 -> 0.34 (195 G/s; issue 72 % active, 145 instructions per 32 samples), against the FP32 cells'
+// six values and index range (8 bytes per weight, 332 instructions); n = 2^26, 2^27 samples: uniform
+// 2.46 -> 1.10, log-normal 2.78 -> 1.80 ms (the grid exceeds L2: random HBM reads again).
+template <uint32_t RNG>
+__global__ __launch_bounds__(kSampleThreads) void k_its_sample_grids(
+    const float* __restrict__ cmf, uint32_t n, const ItsGrid* __restrict__ grids, uint32_t G,
+    uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out) {
+    pdl_entry();
+    const uint64_t s0 =
+        (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * kGridPerThread;
+    if (s0 >= S) return;
+    const uint32_t last = n - 1u;
+    const float total = __ldg(cmf + last);
+    const float scale = pow2f(its_shift(total, G));
+    float t[kGridPerThread];
+    if constexpr (RNG == RNG_REF) {
+        const uint32_t seed32 = static_cast<uint32_t>(seed);
+#pragma unroll
+        for (int v = 0; v < kGridPerThread; ++v)
+            t[v] = search_range_u(cmf, 0, last,
+                                  unit_ref(wang_hash((seed32 ^ 0xA9EC5C80u) +
+                                                     static_cast<uint32_t>(offset + s0 + v))));
+    } else {
+        uint2 ks[10];
+        philox4x32_10_keys(seed, ks);
+#pragma unroll
+        for (int v = 0; v < kGridPerThread; ++v) {
+            const uint64_t g = offset + s0 + v;
+            const uint4 r = philox4x32_10(
+                make_uint4(static_cast<uint32_t>(g), static_cast<uint32_t>(g >> 32), 0u, 0u), ks);
+            t[v] = its_target(r.x, total);
+        }
+    }
+    uint4 lo[kGridPerThread], hi[kGridPerThread];
+    uint32_t F[kGridPerThread], res[kGridPerThread];
+#pragma unroll
+    for (int v = 0; v < kGridPerThread; ++v) {
+        F[v] = grid_f(t[v], scale);
+        ld_block(reinterpret_cast<const uint32_t*>(grids + min(F[v] >> 7, G - 1u)), lo[v], hi[v]);
+    }
+#pragma unroll
+    for (int v = 0; v < kGridPerThread; ++v) {
+        // the first part whose last item's step is not below the target's: the steps do not
+        // decrease, so the word that holds it is found by its last byte (a word is below the
+        // target's step in its last byte exactly when it is below `edge`), the byte in the word
+        // by the borrow-free difference of its bytes (stored as 128 + step)
+        const uint32_t step = F[v] & 127u, edge = (step | 128u) << 24;
+        const uint32_t w6 = hi[v].w | 0xff000000u;
+        const bool up = hi[v].x < edge;                       // words 4 .. 6
+        const uint32_t mid = up ? hi[v].z : lo[v].z;          // word 5 or 1
+        const bool up2 = mid < edge;
+        const uint32_t leaf = up ? (up2 ? w6 : hi[v].y) : (up2 ? lo[v].w : lo[v].y);  // 6 4 2 0
+        const bool up3 = leaf < edge;
+        const uint32_t word = up3 ? (up2 ? (up ? w6 : hi[v].x) : mid) : leaf;
+        const uint32_t r = word - step * 0x01010101u;
+        const uint32_t ge = r & 0x80808080u;
+        const uint32_t in = 4u - __popc(ge);
+        const uint32_t below = (up ? 16u : 0u) + (up2 ? 8u : 0u) + (up3 ? 4u : 0u) + in;
+        const uint32_t e = hi[v].w >> 24;
+        const uint32_t x0 = min(lo[v].x, last);
+        uint32_t x = min(x0 + below, last);
+        // items in the target's own step are told apart by it from 2^23 steps on
+        const bool same = F[v] < (1u << 23) && (r >> (8u * in & 31u) & 0x7fu) == 0u;
+        if (e != 0u) {
+            const uint64_t end = x0 + (static_cast<uint64_t>(same ? kGridSlots + 1u : below + 1u) << e) - 1u;
+            x = static_cast<uint32_t>(min(x0 + (static_cast<uint64_t>(below) << e), static_cast<uint64_t>(last)));
+            uint32_t y = static_cast<uint32_t>(min(end, static_cast<uint64_t>(last)));
+            while (x < y) {
+                const uint32_t mid = x + ((y - x) >> 1);
+                if (t[v] > __ldg(cmf + mid))
+                    x = mid + 1u;
+                else
+                    y = mid;
+            }
+        } else if (same) {
+            while (x < last && t[v] > __ldg(cmf + x)) ++x;
+        }
+        res[v] = x;
+    }
+    if (s0 + kGridPerThread <= S && (reinterpret_cast<uintptr_t>(out) & 7u) == 0) {
+        __stcs(reinterpret_cast<uint2*>(out + s0), make_uint2(res[0], res[1]));
+    } else {
+#pragma unroll
+        for (int v = 0; v < kGridPerThread; ++v)
+            if (s0 + v < S) __stcs(out + s0 + v, res[v]);
+    }
 }
 
 // ---- cells on an FP32 CMF: cells whose targets can meet an inversion ------------------
@@ -1097,7 +1283,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_cells(
     uint4 q0, q1;
     ld_u32x8_policy(reinterpret_cast<const uint32_t*>(cells + k), once, q0, q1);
     // an FP32 CMF's cell may be marked (its targets can meet an inversion, or its start is not
-    // below c_k): bisect those (the compensated CMF's cells are never marked)
+    // below c_k): bisect those
     const bool unsafe = (q0.y & kCellUnsafe) != 0u;
     // (a cell block holds indices < n for the n it was built for; the clamp keeps any other
     // block's search inside the CMF)
@@ -1151,20 +1337,21 @@ __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* 
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
-    const uint32_t x = cell_start_warp(cmf, n, G, group, g, hi);
+    const uint32_t x = cell_start_warp<false>(cmf, n, G, group, g, hi);
     const uint32_t k = g * 32u + (threadIdx.x & 31u);
     if (k < G) guide[k] = x;
 }
 
 // the first two passes: coarse starts, then group starts (scratch: coarse_entries(G) +
 // group_entries(G) words); returns the group array
+template <bool GRID>
 static uint32_t* launch_cell_brackets(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                       uint32_t* scratch) {
     const uint32_t m = coarse_entries(G), ng = group_entries(G);
     uint32_t* group = scratch + m;
-    launch_pdl(k_cell_coarse, (m + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, cmf, n, G,
+    launch_pdl(k_cell_coarse<GRID>, (m + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, cmf, n, G,
                                                                                         scratch);
-    launch_pdl(k_cell_groups, (ng + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, 
+    launch_pdl(k_cell_groups<GRID>, (ng + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, 
         cmf, n, G, scratch, group);
     return group;
 }
@@ -1175,12 +1362,32 @@ static uint32_t warp_blocks(uint32_t G) {
 }
 
 cudaError_t launch_its_cells(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsCell* cells, bool check) {
-    uint32_t* group = launch_cell_brackets(st, cmf, n, G, coarse);
-    if (check)
-        launch_pdl(k_its_cells<true>, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
+                             uint32_t* coarse, ItsCell* cells) {
+    uint32_t* group = launch_cell_brackets<false>(st, cmf, n, G, coarse);
+    launch_pdl(k_its_cells, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_its_grids(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
+                             uint32_t* coarse, ItsGrid* grids) {
+    uint32_t* group = launch_cell_brackets<true>(st, cmf, n, G, coarse);
+    launch_pdl(k_its_grids, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, grids);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_its_sample_grids(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
+                                    const ItsGrid* grids, uint32_t G, uint64_t S, uint64_t seed,
+                                    uint64_t offset, uint32_t* out) {
+    constexpr uint64_t per = kSampleThreads * kGridPerThread;
+    const uint64_t grid = (S + per - 1) / per;
+    if (grid == 0) return cudaSuccess;
+    if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
+    if (rng == RNG_REF)
+        launch_pdl(k_its_sample_grids<RNG_REF>, static_cast<unsigned>(grid), kSampleThreads, 0, st,
+                   cmf, n, grids, G, S, seed, offset, out);
     else
-        launch_pdl(k_its_cells<false>, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
+        launch_pdl(k_its_sample_grids<RNG_PHILOX>, static_cast<unsigned>(grid), kSampleThreads, 0,
+                   st, cmf, n, grids, G, S, seed, offset, out);
     return cudaGetLastError();
 }
 
@@ -1279,7 +1486,7 @@ cudaError_t launch_cutpoint_guide(cudaStream_t st, const float* cmf, uint32_t n,
 
 cudaError_t launch_guide_monotone(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                   uint32_t* coarse, uint32_t* guide) {
-    uint32_t* group = launch_cell_brackets(st, cmf, n, G, coarse);
+    uint32_t* group = launch_cell_brackets<false>(st, cmf, n, G, coarse);
     launch_pdl(k_guide_monotone, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, guide);
     return cudaGetLastError();
 }
