@@ -55,6 +55,7 @@ struct wrs_buffers {
     uint32_t tree_n = 0;         // the n the last build stored them for (0: none)
     uint32_t cells_n = 0;        // the n the last build wrote them for (0: none)
     bool cells_grid = false;     // the last build wrote the grid
+    uint32_t monotone_n = 0;     // the n the last build wrote a compensated CMF for (0: none)
     AliasBlock* blocks = nullptr;  // alias: the table's alias blocks (kBlockMinN < n)
     uint32_t* classes = nullptr;   // the partition's heavy bits, for the blocks
     uint32_t blocks_n = 0;         // the n the last build wrote the alias blocks for (0: none)
@@ -334,6 +335,7 @@ wrs_status wrs_prefix_sum(const wrs_handle* h, void* stream, const float* in, ui
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
+    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
     WRS_CUDA(launch_scan(as_stream(stream), h->cfg.scan_precision != WRS_SCAN_FP32, in, n,
                          out, b->ctrl, b->scan_states, b->cap_tiles, b->partials),
              "prefix sum");
@@ -411,6 +413,7 @@ wrs_status wrs_prefix_sum_blockwise(const wrs_handle* h, void* stream, const flo
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
+    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
     WRS_CUDA(launch_prefix_sum_blockwise(as_stream(stream), in, n, out,
                                          reinterpret_cast<float*>(b->tile_scratch)),
              "block-wise prefix sum");
@@ -540,12 +543,14 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
     const cudaStream_t st = as_stream(stream);
     const bool comp = compensated(h);
     if (h->cfg.method != WRS_METHOD_ALIAS_TABLE) {
+        b->monotone_n = 0;
         WRS_CUDA(launch_scan(st, comp, weights, n, b->cmf, b->ctrl, b->scan_states, b->cap_tiles,
                              b->partials),
                  "ITS build");
         // the compensated CMF is exactly non-decreasing: the galloping construction gives
         // the bisection's entries
         const uint32_t G = guide_entries(n, h->cfg.guiding_entry_size);
+        if (comp) b->monotone_n = n;
         if (h->cfg.method == WRS_METHOD_CUTPOINT)
             WRS_CUDA(comp ? launch_guide_monotone(st, b->cmf, n, G, b->coarse, b->guide)
                           : launch_cutpoint_guide(st, b->cmf, n, G, b->guide),
@@ -664,8 +669,18 @@ wrs_status wrs_sample_at(const wrs_handle* h, void* stream, const wrs_buffers* b
         }
         return wrs_its_sample(h, stream, b->cmf, n, s, seed, offset, samples);
     }
-    if (h->cfg.method == WRS_METHOD_CUTPOINT)
+    if (h->cfg.method == WRS_METHOD_CUTPOINT) {
+        if (b->monotone_n == n && s) {
+            // the compensated CMF does not decrease: the bisection's index is a count
+            if (!samples) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
+            WRS_CUDA(launch_cutpoint_sample(as_stream(stream), h->cfg.rng, b->cmf, n, b->guide,
+                                            guide_entries(n, h->cfg.guiding_entry_size), s, seed,
+                                            offset, samples, true),
+                     "cutpoint sample");
+            return WRS_OK;
+        }
         return wrs_cutpoint_sample(h, stream, b->cmf, n, b->guide, s, seed, offset, samples);
+    }
     if (b->blocks && b->blocks_n == n && s) {
         // the table's alias blocks, written by the last build for this n: the same samples with
         // the table read only where a block does not decide
@@ -702,6 +717,7 @@ wrs_status wrs_test_prefix_sum_stalled(const wrs_handle* h, void* stream, const 
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
+    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
     if (spin_limit == 0 || spin_limit > kSpinLimit)
         return fail(WRS_ERR_INVALID_ARG, "spin_limit out of range");
     const cudaStream_t st = as_stream(stream);

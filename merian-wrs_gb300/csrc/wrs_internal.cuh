@@ -348,9 +348,10 @@ cudaError_t launch_its_sample_grids(cudaStream_t st, uint32_t rng, const float* 
 // tile_scratch: 2 * tiles_for(n) floats; bad: a device word (set when every cell is marked)
 cudaError_t launch_its_marks(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                              ItsCell* cells, float* tile_scratch, uint32_t* bad);
+// monotone: the CMF is known not to decrease
 cudaError_t launch_cutpoint_sample(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
                                    const uint32_t* guide, uint32_t G, uint64_t S, uint64_t seed,
-                                   uint64_t offset, uint32_t* out);
+                                   uint64_t offset, uint32_t* out, bool monotone = false);
 
 // batched forms (one launch each for all distributions of the batch)
 cudaError_t launch_batch_maps(cudaStream_t st, const DistDesc* dist, uint32_t count,
