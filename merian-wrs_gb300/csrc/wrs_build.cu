@@ -153,6 +153,7 @@ __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __rest
         ctrl->mean = m;
         ctrl->mean_lo = __double2float_rn(__dsub_rn(m64, static_cast<double>(m)));
         ctrl->mass_done = 0u;
+        ctrl->block_reads = 0ull;  // the alias blocks of this build add to it
     }
 }
 

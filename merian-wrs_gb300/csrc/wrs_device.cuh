@@ -25,13 +25,20 @@ constexpr uint32_t kSpinLimit = 1u << 21;  // lookback polls before giving up (>
 constexpr uint32_t kCopyDrainLimit = 1u << 25;
 
 // Programmatic dependent launch.  A kernel launched with programmatic stream serialization
-// (launch_pdl) may be scheduled while the kernel before it in the stream still runs: its CTAs
-// wait here until that kernel has completed and its memory is visible, so the launch and the
-// CTAs' start overlap the predecessor's tail instead of following it.  The kernel then lets its
-// own dependent be scheduled.  For an ordinary launch both instructions do nothing.
+// (launch_pdl) may be scheduled while the kernel before it in the stream still runs:
+// its CTAs wait here until that kernel has completed and its memory is visible, so the launch and the
+// CTAs' start overlap the predecessor's tail instead of following it.  A kernel of a build whose grid
+// is about one wave then lets its own dependent be scheduled at once; a larger one's is as its last
+// CTAs end, since CTAs that wait from early on take room from its own (a 2^26-weight build with every
+// grid letting its dependent start at once 1200 us, none of the larger ones 1130, when the others
+// were launched plainly; letting it before a CTA's write-out 951, as it ends 937).  A sampler only
+// waits: the test of the grid's size is 1 % of its instructions.  For an ordinary launch the
+// instructions do nothing.
+constexpr uint32_t kPdlMaxGrid = 2048;
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_entry() {
-    asm volatile("griddepcontrol.wait;" ::: "memory");
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    pdl_wait();
+    if (gridDim.x <= kPdlMaxGrid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // ---------------------------------------------------------------------------

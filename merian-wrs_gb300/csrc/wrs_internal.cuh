@@ -113,17 +113,12 @@ struct BatchView {
     int2* descent;               // per split-pack CTA: the shared top of its bisections
 };
 
-// Grids up to this many CTAs (about one wave of 256-thread CTAs on the device) are launched
-// with programmatic stream serialization; larger ones are launched plainly.  Measured on
-// GB300: the small configuration's per-call build takes 20.2 us with it against 24.6 us
-// without and its sampling 6.3 against 8.2 us, while a build of 2^26 weights takes 1.20
-// against 1.13 ms and a batch graph of 4096 distributions 15.8 against 10.8 ms -- the early
-// scheduled CTAs of a many-wave kernel cost more than the launch gap they hide.
-constexpr uint64_t kPdlMaxGrid = 2048;
-
-// Launches `kernel` (which starts with pdl_entry()) with programmatic stream serialization
-// when its grid is at most kPdlMaxGrid CTAs: it may then be scheduled before its predecessor
-// in the stream has finished.
+// Launches `kernel` (which starts with pdl_entry() or pdl_wait()) with programmatic stream
+// serialization: it may be scheduled before its predecessor in the stream has finished (when it has
+// let it be, or as its last CTAs end).  Measured against overlapping only grids of up to 2048 CTAs
+// (which then all let their dependents be scheduled at once): a 2^26-weight float-float build 972 ->
+// 937 us, a batch of 1024 distributions 772 -> 759 us, 512 served requests 1120 -> 1000 us, the small
+// configuration's pass 25.6 -> 25.5 us.
 template <class... KArgs, class... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
                               cudaStream_t st, Args&&... args) {
@@ -136,8 +131,7 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    const uint64_t ctas = static_cast<uint64_t>(grid.x) * grid.y * grid.z;
-    cfg.numAttrs = ctas <= kPdlMaxGrid ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
 }
 
@@ -223,7 +217,7 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
                                 const AliasBlock* blocks, const unsigned long long* reads,
                                 uint32_t n, uint64_t s, uint64_t seed, uint64_t offset,
                                 uint32_t* out);
-// the blocks of table[0, n) and, into *reads (zeroed first, on the stream), 8 times the entry
+// the blocks of table[0, n) and, into *reads (zero: k_total_mass clears it), 8 times the entry
 // reads one sample of every bucket would cost; classes: the partition's heavy bits
 cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint32_t* classes,
                                 uint32_t n, AliasBlock* blocks, unsigned long long* reads);

@@ -192,7 +192,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_alias_sample(
     const uint2* __restrict__ table, const AliasBlock* __restrict__ blocks,
     const unsigned long long* __restrict__ reads, uint32_t n, uint64_t S, uint64_t seed,
     uint64_t offset, uint32_t coop, uint32_t* __restrict__ out) {
-    pdl_entry();
+    pdl_wait();
     bool use = false;
     if constexpr (BLOCKS) use = __ldg(reads) <= static_cast<unsigned long long>(kBlockMaxReads) * n;
     alias_block<RNG, COOP, BLOCKS, BLOCKS ? kBlockPerThread : kAliasPerThread>(table, blocks, use, n, S, seed, offset, coop, out, blockIdx.x);
@@ -204,7 +204,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_alias_sample(
 template <uint32_t RNG, bool COOP>
 __global__ __launch_bounds__(kSampleThreads) void k_alias_sample_batch(BatchView bv,
                                                                        uint32_t coop) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t d = __ldg(bv.sample_map + blockIdx.x);
     const DistDesc* D = bv.dist + d;
     alias_block<RNG, COOP, false>(D->table, nullptr, false, D->n, D->s, D->seed, 0ull, coop,
@@ -398,7 +398,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample(const float* __re
                                                                uint64_t seed, uint64_t offset,
                                                                uint32_t coop,
                                                                uint32_t* __restrict__ out) {
-    pdl_entry();
+    pdl_wait();
     const uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if constexpr (COOP == 0) {
         if (s >= S) return;
@@ -545,7 +545,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_tree(const float*
                                                                     uint32_t* __restrict__ out,
                                                                     const TreeBlock* __restrict__ blocks,
                                                                     uint32_t B) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float s_tree[kItsTreeNodes];
     const uint32_t last = n - 1u;
     for (uint32_t k = threadIdx.x + 1; k < kItsTreeNodes; k += blockDim.x) {
@@ -949,7 +949,7 @@ template <uint32_t RNG>
 __global__ __launch_bounds__(kSampleThreads) void k_its_sample_grids(
     const float* __restrict__ cmf, uint32_t n, const ItsGrid* __restrict__ grids, uint32_t G,
     uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out) {
-    pdl_entry();
+    pdl_wait();
     const uint64_t s0 =
         (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) * kGridPerThread;
     if (s0 >= S) return;
@@ -1243,7 +1243,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_cells(
     const float* __restrict__ cmf, uint32_t n, const ItsCell* __restrict__ cells, uint32_t G,
     uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out,
     const TreeBlock* __restrict__ blocks, uint32_t L) {
-    pdl_entry();
+    pdl_wait();
     const uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const uint32_t last = n - 1u;
@@ -1448,7 +1448,7 @@ template <uint32_t RNG>
 __global__ __launch_bounds__(kSampleThreads) void k_cutpoint_sample(
     const float* __restrict__ cmf, uint32_t n, const uint32_t* __restrict__ guide, uint32_t G,
     uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out) {
-    pdl_entry();
+    pdl_wait();
     const uint64_t s = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (s >= S) return;
     const uint64_t g = offset + s, g0 = offset + (s & ~31ull);
@@ -1517,7 +1517,7 @@ template <uint32_t RNG>
 __global__ __launch_bounds__(kSampleThreads) void k_cutpoint_sample_mono(
     const float* __restrict__ cmf, uint32_t n, const uint32_t* __restrict__ guide, uint32_t G,
     uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out) {
-    pdl_entry();
+    pdl_wait();
     __shared__ uint4 s_range[kSampleThreads / 32][kCutGroups];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint64_t base = (static_cast<uint64_t>(blockIdx.x) * (kSampleThreads / 32) + warp) * (kCutGroups * 32u);
@@ -1644,8 +1644,6 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
 
 cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint32_t* classes,
                                 uint32_t n, AliasBlock* blocks, unsigned long long* reads) {
-    cudaError_t e = cudaMemsetAsync(reads, 0, sizeof(*reads), st);
-    if (e != cudaSuccess) return e;
     constexpr uint32_t span = kBlockBuildThreads * 32u;  // entries per CTA
     launch_pdl(k_alias_blocks, static_cast<unsigned>((static_cast<uint64_t>(n) + span - 1) / span),
                kBlockBuildThreads, 0, st, table, classes, n, blocks, reads);
