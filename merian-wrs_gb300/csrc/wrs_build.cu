@@ -1219,8 +1219,9 @@ __device__ __forceinline__ void compute_split(const PackIn& c, uint32_t nsplit, 
 // FF: an FP32 pre-test decides most levels without the low words.  d = (h + l) - t differs
 // from the float-float value (h + hl) + (l + ll) - (t + tl) by at most 3u(h + l) + 2u t
 // (u = 2^-24, |lo| <= u |hi|), and the float-float evaluation is accurate to O(u^2); beyond
-// 8u(h + l + t) both have d's sign, so the low words are only read near the split point and
-// every decision is the float-float one.
+// 8u(h + l + t) both have d's sign.  24u t is no less than that while h + l <= 2t, and above d > t
+// is itself decisive, so one margin per split serves: the low words are only read near the split
+// point and every decision is the float-float one.
 template <bool R64, bool FF>
 __device__ __forceinline__ void bisect_one(const PackIn& c, uint32_t nsplit, bool on, uint32_t& io,
                                            uint32_t& jo, float& spill, int a, int b) {
@@ -1228,21 +1229,19 @@ __device__ __forceinline__ void bisect_one(const PackIn& c, uint32_t nsplit, boo
     const float target = __fmul_rn(c.mean, __uint2float_rn(nsplit));
     ff tff{0.f, 0.f};
     if constexpr (FF) tff = ff_target(c.mean, c.mean_lo, nsplit);
+    const float m = __fmul_rn(1.430511474609375e-06f, tff.hi);  // 24u t
     const uint32_t lcm1 = c.lcap;
     while (a <= b) {
         const uint32_t j = static_cast<uint32_t>(a + ((b - a) >> 1));
-        const uint32_t i = j > nsplit ? lcm1 : min(nsplit - j, lcm1);
+        const uint32_t i = min(nsplit - j, lcm1);  // (j > nsplit wraps above any light count)
         const float heavy = j ? __ldg(c.prefix + j - 1) : 0.f;
         const float light = i ? __ldg(c.prefix + c.n - i) : 0.f;
         bool le;
         if constexpr (FF) {
             const float hs = __fadd_rn(heavy, light);
             const float d = __fsub_rn(hs, tff.hi);
-            const float m = __fmul_rn(4.76837158203125e-07f, __fadd_rn(hs, tff.hi));
-            if (d > m) {
-                le = false;
-            } else if (d < -m) {
-                le = true;
+            if (fabsf(d) > m) {
+                le = d < 0.0f;
             } else {
                 const float hl = j ? __ldg(c.prefix_lo + j - 1) : 0.f;
                 const float ll = i ? __ldg(c.prefix_lo + c.n - i) : 0.f;
@@ -1582,34 +1581,36 @@ __device__ void pack_staged(const PackIn& c, const EntryStage& st, uint2* __rest
 // pack_staged for a subproblem whose items all lie inside the staged ranges, inside the heavy
 // and light ranges (j1 <= heavyCount, i1 <= the light count) and that no later subproblem in
 // the window covers: every step is owned and staged, and the end tests reduce to j == j1 and
-// i == i1.  Decisions, arithmetic and staged words are pack_staged's.
+// i == i1.  Decisions, arithmetic and staged words are pack_staged's.  The successor of the stream
+// that advanced is loaded without a test: heavy position j + 1 <= heavyCount and light rank
+// i <= the light count are positions of the partition.
+template <bool ELEMS>
 __device__ __forceinline__ void pack_staged_fast(const PackIn& c, const EntryStage& st,
                                                  uint32_t i0, uint32_t i1, uint32_t j0,
                                                  uint32_t j1, float spill) {
-    uint32_t i = i0, j = j0;
+    auto weight_at = [&](uint32_t pos) { return ELEMS ? __ldg(c.elems + pos) : item_weight(c, pos); };
+    // staged word of heavy position j: st.w[j - h0]; of light rank i: st.w[q - h0], q = i + to_q
+    const uint32_t to_q = st.h0 + st.hcnt - st.l0, q1 = i1 + to_q, light_pos = c.n - 1u + to_q;
+    uint32_t* const w = st.w - st.h0;
+    uint32_t j = j0, q = i0 + to_q;
+    if (j == j1 && q == q1) return;
     float wv = spill;
-    const bool close_last = c.lcap == c.lc;
-    if (wv == 0.0f && (i < i1 || j < j1)) wv = item_weight(c, j);
-    float next_h = j < j1 ? item_weight(c, j + 1u) : 0.f;
-    float next_l = i < i1 ? item_weight(c, c.n - 1u - i) : 0.f;
-    uint32_t* const wh = st.w - st.h0;             // heavy position j -> its word
-    uint32_t* const wl = st.w + st.hcnt - st.l0;   // light rank i -> its word
-    while (i < i1 || j < j1) {
-        const bool heavy_step = j != j1 && (i == i1 || wv <= c.mean);
+    if (wv == 0.0f) wv = weight_at(j);
+    if (wv != wv) wv = __uint_as_float(0x7fffffffu);  // (a weight's NaN; sums' are this one)
+    const uint32_t jmax = c.lcap == c.lc ? c.hc - 1u : c.hc;  // the current heavy's last position
+    float next_h = weight_at(j + 1u <= c.hc ? j + 1u : c.hc);
+    float next_l = weight_at(light_pos - q);
+    do {
+        const bool heavy_step = j != j1 && (q == q1 || wv <= c.mean);
         const float weight = heavy_step ? next_h : next_l;
-        const uint32_t J = close_last && j >= c.hc ? c.hc - 1u : j;
-        if (heavy_step)
-            wh[j] = wv != wv ? 0x7fffffffu : __float_as_uint(wv);
-        else
-            wl[i] = J;
+        w[heavy_step ? j : q] = heavy_step ? __float_as_uint(wv) : min(j, jmax);
         j += heavy_step ? 1u : 0u;
-        i += heavy_step ? 0u : 1u;
-        const bool more = heavy_step ? j < j1 : i < i1;
-        const float nw = more ? item_weight(c, heavy_step ? j + 1u : c.n - 1u - i) : 0.f;
+        q += heavy_step ? 0u : 1u;
+        const float nw = weight_at(heavy_step ? min(j + 1u, c.hc) : light_pos - q);
         next_h = heavy_step ? nw : next_h;
         next_l = heavy_step ? next_l : nw;
         wv = __fsub_rn(__fadd_rn(wv, weight), c.mean);
-    }
+    } while (j != j1 || q != q1);
 }
 
 struct SplitArgs {
@@ -1672,6 +1673,14 @@ __global__ __launch_bounds__(kDescentThreads) void k_split_descent(SplitArgs a, 
 }
 
 
+// Bound by instruction issue (60 % active) and the L1's wavefronts (69 %) together; 146 instructions
+// per weight in the float-float form, where it took 224.  n = 2^26, split size 12: 0.500 -> 0.415 ms
+// uniform, 0.321 -> 0.272 ms log-normal(0, 3) with outliers, against walks and a write-out that
+// marked and tested every staged word, margins recomputed per level and four positions per thread
+// in the write-out's last, mostly empty round.  Walks on weights staged in shared memory (0.493 /
+// 0.352) and bisections that share levels per warp (slower too) lose more to their barriers and
+// rounds than they save in accesses.
+//
 // Slot t of CTA b (t < kSplitSlots; thread t % kSplitThreads holds slots t and t + 512) holds
 // split k = b*kSplitPack + t (k in [0, K]) and packs subproblem k = [split_k, split_{k+1})
 // for t < kSplitPack, k < K; split_{k+1} comes from the next slot through shared memory
@@ -1681,7 +1690,6 @@ template <bool R64, bool FF, bool BATCH, bool RECORDS = false>
 __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, BatchView bv) {
     pdl_entry();
     __shared__ uint32_t s_i[kSplitSlots], s_j[kSplitSlots];
-    __shared__ float s_spill[kSplitSlots];
     const float* w = a.w;
     uint32_t n = a.n;
     const BuildCtrl* ctrl = a.ctrl;
@@ -1753,7 +1761,6 @@ __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, Ba
         const int slot = threadIdx.x + v * kSplitThreads;
         s_i[slot] = si[v];
         s_j[slot] = sj[v];
-        s_spill[slot] = sp[v];
     }
     __syncthreads();
     // stage the items of this CTA's subproblems [split_kb, split_{kb + npack}) when the launch
@@ -1767,53 +1774,112 @@ __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, Ba
         const uint32_t npack = min(static_cast<uint32_t>(kSplitPack), K - kb);
         constexpr uint32_t kMargin = 64;
         EntryStage es{reinterpret_cast<uint32_t*>(s_items), s_j[0], 0u, s_i[0], 0u};
-        const uint32_t hext = (s_j[npack] > es.h0 ? s_j[npack] - es.h0 : 0u) + kMargin;
-        const uint32_t lext = (s_i[npack] > es.l0 ? s_i[npack] - es.l0 : 0u) + kMargin;
-        if (hext + lext <= stage_entries_for(a.split_size)) {
-            es.hcnt = hext;
-            es.lcnt = lext;
-        }
+        const uint32_t stage = stage_entries_for(a.split_size);
+        const uint32_t hspan = s_j[npack] > es.h0 ? s_j[npack] - es.h0 : 0u;
+        const uint32_t lspan = s_i[npack] > es.l0 ? s_i[npack] - es.l0 : 0u;
         // the CTA's splits in slot order never step back (the common case): then no later
         // subproblem covers an earlier one's items, and the ownership window is not consulted
-        bool mono = true;
-#pragma unroll
-        for (int v = 0; v < kSplitPerThread; ++v) {
-            const int t = threadIdx.x + v * kSplitThreads;
-            if (t + 1 < kSplitSlots) mono = mono && s_i[t + 1] >= s_i[t] && s_j[t + 1] >= s_j[t];
-        }
-        for (uint32_t q = threadIdx.x; q < es.hcnt + es.lcnt; q += blockDim.x) es.w[q] = kNotStaged;
-        const bool all_mono = __syncthreads_and(mono);
-#pragma unroll 1
-        for (int v = 0; v < kSplitPerThread; ++v) {
-            const int t = threadIdx.x + v * kSplitThreads;
-            const uint32_t k = kv[v];
-            if (t >= kSplitPack || k >= K) continue;
-            const uint32_t i1 = max(s_i[t + 1], si[v]), j1 = max(s_j[t + 1], sj[v]);
-            bool clean = true;
-            int count = 0;
-            if (!all_mono) {
-                count = static_cast<int>(min(static_cast<uint32_t>(kSplitLook), K - 1u - k));
-                for (int d = 1; d <= count; ++d)
-                    clean = clean && s_i[t + d] >= i1 && s_j[t + d] >= j1;
-                if (k + kSplitLook + 1u < K &&
-                    (s_i[t + kSplitLook + 1] < i1 || s_j[t + kSplitLook + 1] < j1))
-                    atomicOr(a.status, kStatusNonMonotone);
-            }
-            const LaterSplits later{s_i, s_j, t, count};
-            const bool inside = sj[v] >= es.h0 && j1 - es.h0 <= es.hcnt && si[v] >= es.l0 &&
-                                i1 - es.l0 <= es.lcnt && j1 <= c.hc && i1 <= c.lc;
-            if (clean && inside)
-                pack_staged_fast(c, es, si[v], i1, sj[v], j1, sp[v]);
+        const int slot1 = min(static_cast<int>(threadIdx.x) + 1, kSplitSlots - 1);
+        const uint32_t i_next = s_i[slot1], j_next = s_j[slot1];
+        const bool all_mono = __syncthreads_and(i_next >= si[0] && j_next >= sj[0]);
+        auto walk = [&](uint32_t i0, uint32_t i1, uint32_t j0, uint32_t j1, float spill) {
+            if (c.elems)
+                pack_staged_fast<true>(c, es, i0, i1, j0, j1, spill);
             else
-                pack_staged(c, es, table, si[v], i1, sj[v], j1, sp[v], clean ? nullptr : &later);
+                pack_staged_fast<false>(c, es, i0, i1, j0, j1, spill);
+        };
+        // then, and within the heavy and light ranges, the CTA packs each position of [h0, h0 + hspan)
+        // and each rank of [l0, l0 + lspan) once: no word has to be marked, none to be tested
+        const bool exact = all_mono && s_j[npack] <= c.hc && s_i[npack] <= c.lc && hspan + lspan <= stage;
+        if (exact) {
+            es.hcnt = hspan;
+            es.lcnt = lspan;
+            if (threadIdx.x < kSplitPack && kv[0] < K) walk(si[0], i_next, sj[0], j_next, sp[0]);
+        } else {
+            // with a margin for splits stepping back at the end; staged only if both fit
+            if (hspan + lspan + 2u * kMargin <= stage) {
+                es.hcnt = hspan + kMargin;
+                es.lcnt = lspan + kMargin;
+            }
+            for (uint32_t q = threadIdx.x; q < es.hcnt + es.lcnt; q += blockDim.x)
+                es.w[q] = kNotStaged;
+            __syncthreads();
+#pragma unroll 1
+            for (int v = 0; v < kSplitPerThread; ++v) {
+                const int t = threadIdx.x + v * kSplitThreads;
+                const uint32_t k = kv[v];
+                if (t >= kSplitPack || k >= K) continue;
+                const uint32_t i1 = max(s_i[t + 1], si[v]), j1 = max(s_j[t + 1], sj[v]);
+                bool clean = true;
+                int count = 0;
+                if (!all_mono) {
+                    count = static_cast<int>(min(static_cast<uint32_t>(kSplitLook), K - 1u - k));
+                    for (int d = 1; d <= count; ++d)
+                        clean = clean && s_i[t + d] >= i1 && s_j[t + d] >= j1;
+                    if (k + kSplitLook + 1u < K &&
+                        (s_i[t + kSplitLook + 1] < i1 || s_j[t + kSplitLook + 1] < j1))
+                        atomicOr(a.status, kStatusNonMonotone);
+                }
+                const LaterSplits later{s_i, s_j, t, count};
+                const bool inside = sj[v] >= es.h0 && j1 - es.h0 <= es.hcnt && si[v] >= es.l0 &&
+                                    i1 - es.l0 <= es.lcnt && j1 <= c.hc && i1 <= c.lc;
+                if (clean && inside)
+                    walk(si[v], i1, sj[v], j1, sp[v]);
+                else
+                    pack_staged(c, es, table, si[v], i1, sj[v], j1, sp[v], clean ? nullptr : &later);
+            }
         }
         __syncthreads();
         // write-out: consecutive lanes on consecutive positions, kOutBatch positions per thread
         // with their loads in flight together (write_heavy / write_light's values; positions
         // clamped into [0, n) so that every load is in bounds, only staged entries stored)
         const bool close_last = c.lcap == c.lc;
-        constexpr int kOutBatch = 4;
-        const uint32_t bd = blockDim.x, nm1 = c.n - 1u;
+        constexpr int kOutBatch = 3;  // (2 and 4: 442 us where 3 takes 415, uniform n = 2^26)
+        const uint32_t bd = kSplitThreads, nm1 = c.n - 1u;
+        if (exact && c.elems && !(close_last && es.h0 + es.hcnt == c.hc)) {
+            // every word is staged, every position and its successor lie in the partition
+            const uint32_t* const hidx = c.idx + es.h0;
+            for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
+                uint32_t t[kOutBatch], al[kOutBatch];
+                float r[kOutBatch];
+#pragma unroll
+                for (int u = 0; u < kOutBatch; ++u) {
+                    const uint32_t q = q0 + u * bd;
+                    t[u] = c.n;
+                    if (q < es.hcnt) {
+                        r[u] = __uint_as_float(es.w[q]);
+                        t[u] = __ldg(hidx + q);
+                        al[u] = __ldg(hidx + q + 1u);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kOutBatch; ++u)
+                    if (t[u] < c.n)
+                        table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(r[u], c.mean)), al[u]);
+            }
+            const uint32_t* const lidx = c.idx + (nm1 - es.l0);
+            const float* const lelem = c.elems + (nm1 - es.l0);
+            const uint32_t* const lw = es.w + es.hcnt;
+            for (uint32_t q0 = threadIdx.x; q0 < es.lcnt; q0 += kOutBatch * bd) {
+                uint32_t t[kOutBatch], aj[kOutBatch];
+                float wt[kOutBatch];
+#pragma unroll
+                for (int u = 0; u < kOutBatch; ++u) {
+                    const uint32_t q = q0 + u * bd;
+                    t[u] = c.n;
+                    if (q < es.lcnt) {
+                        t[u] = __ldg(lidx - q);
+                        wt[u] = __ldg(lelem - q);
+                        aj[u] = __ldg(c.idx + lw[q]);
+                    }
+                }
+#pragma unroll
+                for (int u = 0; u < kOutBatch; ++u)
+                    if (t[u] < c.n)
+                        table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(wt[u], c.mean)), aj[u]);
+            }
+            return;
+        }
         for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
             uint32_t r[kOutBatch], t[kOutBatch], al[kOutBatch];
 #pragma unroll
