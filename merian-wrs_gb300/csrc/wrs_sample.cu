@@ -1624,8 +1624,11 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
     if (ctas == 0) return cudaSuccess;
     if (ctas > 0x7fffffffull) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(ctas));
+    // (through the blocks it follows k_alias_blocks, which has no shared memory)
+    const bool overlap = b || ctas <= kPdlMaxGrid;
     auto go = [&](auto kernel) {
-        launch_pdl(kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed, offset, coop, out);
+        launch_overlapped(overlap, kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed,
+                          offset, coop, out);
     };
     if (rng == RNG_REF) {
         if (coop)
@@ -1653,13 +1656,17 @@ cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint3
 cudaError_t launch_batch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop,
                                       const BatchView& b) {
     if (b.sample_blocks == 0) return cudaSuccess;
+    auto go = [&](auto kernel, uint32_t c) {
+        launch_overlapped(b.sample_blocks <= kPdlMaxGrid, kernel, b.sample_blocks, kSampleThreads, 0, st,
+                          b, c);
+    };
     if (rng == RNG_REF) {
         if (coop)
-            launch_pdl(k_alias_sample_batch<RNG_REF, true>, b.sample_blocks, kSampleThreads, 0, st, b, coop);
+            go(k_alias_sample_batch<RNG_REF, true>, coop);
         else
-            launch_pdl(k_alias_sample_batch<RNG_REF, false>, b.sample_blocks, kSampleThreads, 0, st, b, 0u);
+            go(k_alias_sample_batch<RNG_REF, false>, 0u);
     } else {
-        launch_pdl(k_alias_sample_batch<RNG_PHILOX, false>, b.sample_blocks, kSampleThreads, 0, st, b, 0u);
+        go(k_alias_sample_batch<RNG_PHILOX, false>, 0u);
     }
     return cudaGetLastError();
 }
