@@ -10,6 +10,7 @@
 //                       outputs (after k_total_mass, which sets the grid)
 //   k_split_pack        PSA split search + pack, one thread per split
 //                                                          (src/device/wrs/alias/psa/splitpack/inline/shader.comp)
+//   k_build_small       those of a small distribution in one launch: a cluster of up to eight CTAs
 //
 // The total-mass, partition and split+pack kernels come in two forms from one body: a
 // single distribution (BATCH = false; CTA b works on tile / split block b), and a batch
@@ -89,6 +90,33 @@ __device__ __forceinline__ uint32_t park_slot(uint32_t q) { return q ^ ((q >> 3)
 // stored in FP64, and the last tile of the distribution to finish sums the partials in FP64
 // in a fixed order.  The total is therefore a function of the weights alone (not of the
 // launch geometry, of the buffer's alignment or of other distributions in a batch).
+__device__ __forceinline__ void tile_mass_warp(const float (&x)[4][4], ff* s_part) {
+    ff acc = {0.0f, 0.0f};
+#pragma unroll
+    for (int v = 0; v < 4; ++v)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc = carry_add<true>(acc, ff{x[v][c], 0.0f});
+    acc = ff_warp_total(acc);
+    if ((threadIdx.x & 31u) == 0u) s_part[threadIdx.x >> 5] = acc;
+}
+__device__ __forceinline__ double tile_mass(const ff* s_part) {
+    ff b = s_part[0];
+    for (int k = 1; k < kTileWarps; ++k) b = carry_add<true>(b, s_part[k]);
+    return __dadd_rn(static_cast<double>(b.hi), static_cast<double>(b.lo));
+}
+// the mean as FP64 and as a float-float pair
+struct Mean {
+    double m64;
+    float hi, lo;
+};
+__device__ __forceinline__ Mean mean_of(double total, uint32_t n) {
+    Mean m;
+    m.m64 = n ? __ddiv_rn(total, static_cast<double>(n)) : 0.0;
+    m.hi = __double2float_rn(m.m64);
+    m.lo = __double2float_rn(__dsub_rn(m.m64, static_cast<double>(m.hi)));
+    return m;
+}
+
 template <bool BATCH>
 __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __restrict__ w_in,
                                                              uint32_t n_in,
@@ -114,20 +142,11 @@ __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __rest
     const uint32_t lt = tile - first, ntiles = tiles_for(n);
     float x[4][4];
     load_tile(w, n, lt, x);
-    ff acc = {0.0f, 0.0f};
-#pragma unroll
-    for (int v = 0; v < 4; ++v)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc = carry_add<true>(acc, ff{x[v][c], 0.0f});
-
-    acc = ff_warp_total(acc);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    if (lane == 0) s_part[warp] = acc;
+    tile_mass_warp(x, s_part);
     __syncthreads();
     if (threadIdx.x == 0) {
-        ff b = s_part[0];
-        for (int k = 1; k < kTileWarps; ++k) b = carry_add<true>(b, s_part[k]);
-        partials[tile] = __dadd_rn(static_cast<double>(b.hi), static_cast<double>(b.lo));
+        partials[tile] = tile_mass(s_part);
         __threadfence();
         const uint32_t prev = atomicAdd(&ctrl->mass_done, 1u);
         s_last = (prev == ntiles - 1u);
@@ -146,12 +165,11 @@ __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __rest
     if (threadIdx.x == 0) {
         double total = 0.0;
         for (int k = 0; k < kTileWarps; ++k) total = __dadd_rn(total, s_red[k]);
+        const Mean m = mean_of(total, n);
         ctrl->total = total;
-        const double m64 = n ? __ddiv_rn(total, static_cast<double>(n)) : 0.0;
-        const float m = __double2float_rn(m64);
-        ctrl->mean64 = m64;
-        ctrl->mean = m;
-        ctrl->mean_lo = __double2float_rn(__dsub_rn(m64, static_cast<double>(m)));
+        ctrl->mean64 = m.m64;
+        ctrl->mean = m.hi;
+        ctrl->mean_lo = m.lo;
         ctrl->mass_done = 0u;
         ctrl->block_reads = 0ull;  // the alias blocks of this build add to it
     }
@@ -394,10 +412,28 @@ struct PartArgs {
 // prefix as a float-float pair (prefix[] is its high word): float-float local sums give the
 // carried prefix before each thread's first item, and the thread adds its items to that in
 // float-float.
-template <bool COMP, bool FFOUT, bool BATCH, bool BW = false>
-__global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partition(PartArgs a,
-                                                                                   BatchView bv) {
-    pdl_entry();
+//
+// The carry into a tile comes from the lookback, from precomputed offsets (block-wise), or, where
+// the CTAs of one cluster hold the whole distribution (k_build_small), from the other tiles'
+// aggregates, which the CTAs store into each other's shared memory.
+enum class Carry { kLookback, kGiven, kCluster };
+struct PartAgg {
+    ff h, l;
+    uint32_t c;
+};
+struct ClusterPart {
+    uint32_t rank, tiles, ctas;  // this CTA (its tile), tiles and CTAs of the cluster
+    double total;
+    float mean;
+    PartAgg* agg;       // shared: [tiles], written by the cluster's CTAs
+    uint32_t* heavies;  // shared: the heavy count of the distribution
+};
+constexpr uint32_t kPartBytes = kTileItems * 4 + kStageWords * 2 + kStageWords * 4;
+
+template <bool COMP, bool FFOUT, bool BATCH, Carry CARRY>
+__device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchView& bv,
+                                               unsigned char* s_raw, const ClusterPart& cl) {
+    constexpr bool BW = CARRY == Carry::kGiven, CLUSTER = CARRY == Carry::kCluster;
     // warp totals (phase A), turned into warp-exclusive offsets by warp 0 (phase B)
     __shared__ uint32_t s_wc[kTileWarps];
     __shared__ float s_wh[kTileWarps], s_wl[kTileWarps];  // local FP32 sums (!FFOUT)
@@ -408,7 +444,7 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
     // heavy items take slots [0, heavy) in order, its light items slots 4095, 4094, ... in order,
     // so both runs are written out as contiguous, coalesced segments (stage_idx pads 1 word per
     // 32).  Until phase C the staging area holds the lane-exclusive offsets of phase A.
-    __shared__ __align__(16) unsigned char s_raw[kTileItems * 4 + kStageWords * 2 + kStageWords * 4];
+    // (s_raw: kPartBytes of shared memory)
     float4* const s_x = reinterpret_cast<float4*>(s_raw);
     uint16_t* const s_key = reinterpret_cast<uint16_t*>(s_raw + kTileItems * 4);
     float* const s_val = reinterpret_cast<float*>(s_raw + kTileItems * 4 + kStageWords * 2);
@@ -417,7 +453,9 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
     float2* const s_ll = reinterpret_cast<float2*>(s_val + 3 * kTileThreads);
 
     PartState* cur = nullptr;
-    const uint32_t tile = BW ? blockIdx.x : lookback_begin(a.lb, a.states, a.cap_tiles, cur);
+    const uint32_t tile = CLUSTER ? cl.rank
+                          : BW    ? blockIdx.x
+                                  : lookback_begin(a.lb, a.states, a.cap_tiles, cur);
     const float* w = a.w;
     uint32_t n = a.n, first = 0;
     BuildCtrl* ctrl = a.ctrl;
@@ -430,10 +468,10 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
         ctrl = bv.dctrl + (D - bv.dist);
     }
     const uint32_t lt = tile - first;
-    const float pivot = ctrl->mean;
+    const float pivot = CLUSTER ? cl.mean : ctrl->mean;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-    {
+    if constexpr (!CLUSTER) {  // (a cluster's CTA has parked its tile for the total mass)
         float x[4][4];
         load_tile(w, n, lt, x);
 #pragma unroll
@@ -475,7 +513,7 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
             }
         }
         const uint32_t tc = __popc(heavies);
-        if constexpr (!BATCH && !BW) {
+        if constexpr (!BATCH && CARRY == Carry::kLookback) {
             if (a.classes)
                 a.classes[static_cast<size_t>(lt) * kTileThreads + threadIdx.x] =
                     static_cast<uint16_t>(heavies);
@@ -550,7 +588,10 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
         }
         ff exh{0.f, 0.f}, exl{0.f, 0.f};
         uint32_t exc = 0;
-        if constexpr (BW) {
+        if constexpr (CLUSTER) {
+            if (static_cast<uint32_t>(lane) < cl.ctas)
+                st_cluster(cl.agg + tile, lane, PartAgg{agg_h, agg_l, agg_c});
+        } else if constexpr (BW) {
             exh = {__ldg(a.bw_h + tile), 0.f};
             exl = {__ldg(a.bw_l + tile), 0.f};
             exc = __ldg(a.bw_c + tile);
@@ -596,13 +637,47 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
             exc = ex.c;
         }
         if (lane == 0) {
-            s_exh = exh;
-            s_exl = exl;
-            s_exc = exc;
+            if constexpr (!CLUSTER) {
+                s_exh = exh;
+                s_exl = exl;
+                s_exc = exc;
+            }
             s_aggc = agg_c;
         }
-        if constexpr (!BW)
+        if constexpr (CARRY == Carry::kLookback)
             if (threadIdx.x == 0) left = lookback_leave(a.lb);
+    }
+    if constexpr (CLUSTER) {
+        cluster_arrive();
+        cluster_wait();
+        if (warp == 0) {
+            const PartAgg g = static_cast<uint32_t>(lane) < cl.tiles ? cl.agg[lane] : PartAgg{};
+            const uint32_t hc = __reduce_add_sync(0xffffffffu, g.c);
+            const uint32_t before = __reduce_add_sync(0xffffffffu, static_cast<uint32_t>(lane) < tile ? g.c : 0u);
+            ff exh{0.f, 0.f}, exl{0.f, 0.f};
+            if (tile != 0u) {
+                if constexpr (COMP) {
+                    const int grid = fx_grid(cl.total);
+                    const bool in = static_cast<uint32_t>(lane) < tile;
+                    const PartX ex = part_sum_x(PartX{in ? fx_from_ff(g.h, grid) : 0,
+                                                      in ? fx_from_ff(g.l, grid) : 0, 0u});
+                    // (the words of the lookback: what they cut off a NaN's conversion)
+                    exh = fx_to_ff(fx_unpack(fx_word_lo(ex.h), fx_word_hi(ex.h)), grid);
+                    exl = fx_to_ff(fx_unpack(fx_word_lo(ex.l), fx_word_hi(ex.l)), grid);
+                } else {
+                    for (uint32_t r = 0; r < tile; ++r) {
+                        exh.hi = __fadd_rn(exh.hi, __shfl_sync(0xffffffffu, g.h.hi, r));
+                        exl.hi = __fadd_rn(exl.hi, __shfl_sync(0xffffffffu, g.l.hi, r));
+                    }
+                }
+            }
+            if (lane == 0) {
+                s_exh = exh;
+                s_exl = exl;
+                s_exc = before;
+                *cl.heavies = hc;
+            }
+        }
     }
     __syncthreads();
 
@@ -724,7 +799,16 @@ __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partiti
         }
     }
     if (threadIdx.x == 0 && lt == tiles_for(n) - 1u) ctrl->heavy_count = ex_c + s_aggc;
-    if constexpr (!BW) lookback_end(a.lb, left);
+    if constexpr (CARRY == Carry::kLookback) lookback_end(a.lb, left);
+}
+
+template <bool COMP, bool FFOUT, bool BATCH, bool BW = false>
+__global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partition(PartArgs a,
+                                                                                   BatchView bv) {
+    pdl_entry();
+    __shared__ __align__(16) unsigned char s_raw[kPartBytes];
+    partition_tile<COMP, FFOUT, BATCH, BW ? Carry::kGiven : Carry::kLookback>(a, bv, s_raw,
+                                                                              ClusterPart{});
 }
 
 template <bool BATCH>
@@ -1124,6 +1208,17 @@ struct PackIn {
     uint32_t lcap;  // largest light count a split may take: lc - 1 (shader) or lc
     float mean;
     float mean_lo;  // (mean, mean_lo) = total / N as a float-float pair
+    template <class T>
+    static __device__ __forceinline__ T ld(const T* p) {
+        return __ldg(p);
+    }
+};
+// the same of a partition that the running kernel has written itself
+struct PackOwn : PackIn {
+    template <class T>
+    static __device__ __forceinline__ T ld(const T* p) {
+        return *p;
+    }
 };
 
 // Float-float (FP32) evaluation of sigma - target with sigma = (h + hl) + (l + ll) and
@@ -1212,56 +1307,18 @@ __device__ __forceinline__ void compute_split(const PackIn& c, uint32_t nsplit, 
     jo = j;
 }
 
-// compute_split's probe sequence and arithmetic for the split-pack's one split per thread,
-// started from (a, b): the bisection state after the levels every split of the CTA decides
-// alike (split_descent), or (0, hc - 1) from the top.
-//
-// FF: an FP32 pre-test decides most levels without the low words.  d = (h + l) - t differs
-// from the float-float value (h + hl) + (l + ll) - (t + tl) by at most 3u(h + l) + 2u t
-// (u = 2^-24, |lo| <= u |hi|), and the float-float evaluation is accurate to O(u^2); beyond
-// 8u(h + l + t) both have d's sign.  24u t is no less than that while h + l <= 2t, and above d > t
-// is itself decisive, so one margin per split serves: the low words are only read near the split
-// point and every decision is the float-float one.
-template <bool R64, bool FF>
-__device__ __forceinline__ void bisect_one(const PackIn& c, uint32_t nsplit, bool on, uint32_t& io,
-                                           uint32_t& jo, float& spill, int a, int b) {
-    if (!on) return;
-    const float target = __fmul_rn(c.mean, __uint2float_rn(nsplit));
-    ff tff{0.f, 0.f};
-    if constexpr (FF) tff = ff_target(c.mean, c.mean_lo, nsplit);
-    const float m = __fmul_rn(1.430511474609375e-06f, tff.hi);  // 24u t
+// the split a bisection ends at, with its residual
+template <bool R64, bool FF, class P>
+__device__ __forceinline__ void split_at(const P& c, uint32_t nsplit, float target, ff tff, int b,
+                                         uint32_t& io, uint32_t& jo, float& spill) {
     const uint32_t lcm1 = c.lcap;
-    while (a <= b) {
-        const uint32_t j = static_cast<uint32_t>(a + ((b - a) >> 1));
-        const uint32_t i = min(nsplit - j, lcm1);  // (j > nsplit wraps above any light count)
-        const float heavy = j ? __ldg(c.prefix + j - 1) : 0.f;
-        const float light = i ? __ldg(c.prefix + c.n - i) : 0.f;
-        bool le;
-        if constexpr (FF) {
-            const float hs = __fadd_rn(heavy, light);
-            const float d = __fsub_rn(hs, tff.hi);
-            if (fabsf(d) > m) {
-                le = d < 0.0f;
-            } else {
-                const float hl = j ? __ldg(c.prefix_lo + j - 1) : 0.f;
-                const float ll = i ? __ldg(c.prefix_lo + c.n - i) : 0.f;
-                le = ff_sigma_minus(heavy, hl, light, ll, tff.hi, tff.lo) <= 0.0f;
-            }
-        } else {
-            le = __fadd_rn(light, heavy) <= target;
-        }
-        if (le)
-            a = static_cast<int>(j) + 1;
-        else
-            b = static_cast<int>(j) - 1;
-    }
     const uint32_t j = b < 0 ? 0u : static_cast<uint32_t>(b);
     const uint32_t i = j > nsplit ? lcm1 : min(nsplit - j, lcm1);
-    const float light = i == 0 ? 0.f : __ldg(c.prefix + c.n - i);
-    const float heavy2 = __ldg(c.prefix + j);
+    const float light = i == 0 ? 0.f : c.ld(c.prefix + c.n - i);
+    const float heavy2 = c.ld(c.prefix + j);
     if constexpr (FF) {
-        const float hl2 = __ldg(c.prefix_lo + j);
-        const float l2 = i == 0 ? 0.f : __ldg(c.prefix_lo + c.n - i);
+        const float hl2 = c.ld(c.prefix_lo + j);
+        const float l2 = i == 0 ? 0.f : c.ld(c.prefix_lo + c.n - i);
         spill = ff_sigma_minus(heavy2, hl2, light, l2, tff.hi, tff.lo);
     } else if constexpr (R64) {
         const double target64 =
@@ -1273,6 +1330,119 @@ __device__ __forceinline__ void bisect_one(const PackIn& c, uint32_t nsplit, boo
     }
     io = i;
     jo = j;
+}
+
+// compute_split's probe sequence and arithmetic for the split-pack's one split per thread,
+// started from (a, b): the bisection state after the levels every split of the CTA decides
+// alike (split_descent), or (0, hc - 1) from the top.
+//
+// FF: an FP32 pre-test decides most levels without the low words.  d = (h + l) - t differs
+// from the float-float value (h + hl) + (l + ll) - (t + tl) by at most 3u(h + l) + 2u t
+// (u = 2^-24, |lo| <= u |hi|), and the float-float evaluation is accurate to O(u^2); beyond
+// 8u(h + l + t) both have d's sign.  24u t is no less than that while h + l <= 2t, and above d > t
+// is itself decisive, so one margin per split serves: the low words are only read near the split
+// point and every decision is the float-float one.
+template <bool R64, bool FF, class P>
+__device__ __forceinline__ void bisect_one(const P& c, uint32_t nsplit, bool on, uint32_t& io,
+                                           uint32_t& jo, float& spill, int a, int b) {
+    if (!on) return;
+    const float target = __fmul_rn(c.mean, __uint2float_rn(nsplit));
+    ff tff{0.f, 0.f};
+    if constexpr (FF) tff = ff_target(c.mean, c.mean_lo, nsplit);
+    const float m = __fmul_rn(1.430511474609375e-06f, tff.hi);  // 24u t
+    const uint32_t lcm1 = c.lcap;
+    while (a <= b) {
+        const uint32_t j = static_cast<uint32_t>(a + ((b - a) >> 1));
+        const uint32_t i = min(nsplit - j, lcm1);  // (j > nsplit wraps above any light count)
+        const float heavy = j ? c.ld(c.prefix + j - 1) : 0.f;
+        const float light = i ? c.ld(c.prefix + c.n - i) : 0.f;
+        bool le;
+        if constexpr (FF) {
+            const float hs = __fadd_rn(heavy, light);
+            const float d = __fsub_rn(hs, tff.hi);
+            if (fabsf(d) > m) {
+                le = d < 0.0f;
+            } else {
+                const float hl = j ? c.ld(c.prefix_lo + j - 1) : 0.f;
+                const float ll = i ? c.ld(c.prefix_lo + c.n - i) : 0.f;
+                le = ff_sigma_minus(heavy, hl, light, ll, tff.hi, tff.lo) <= 0.0f;
+            }
+        } else {
+            le = __fadd_rn(light, heavy) <= target;
+        }
+        if (le)
+            a = static_cast<int>(j) + 1;
+        else
+            b = static_cast<int>(j) - 1;
+    }
+    split_at<R64, FF>(c, nsplit, target, tff, b, io, jo, spill);
+}
+
+// bisect_one from the top, three levels per round trip: the midpoints of the seven nodes that the next
+// three levels may probe are read together (k_build_small, whose few splits wait for each load).
+template <bool R64, bool FF, class P>
+__device__ __forceinline__ void bisect_wide(const P& c, uint32_t nsplit, bool on, uint32_t& io,
+                                            uint32_t& jo, float& spill) {
+    if (!on) return;
+    const float target = __fmul_rn(c.mean, __uint2float_rn(nsplit));
+    ff tff{0.f, 0.f};
+    if constexpr (FF) tff = ff_target(c.mean, c.mean_lo, nsplit);
+    const float m = __fmul_rn(1.430511474609375e-06f, tff.hi);  // 24u t
+    const uint32_t lcm1 = c.lcap;
+    int a = 0, b = static_cast<int>(c.hc) - 1;
+    while (a <= b) {
+        int lo[7], hi[7];
+        float heavy[7], light[7];
+        lo[0] = a;
+        hi[0] = b;
+#pragma unroll
+        for (int k = 0; k < 7; ++k) {
+            const int mid = lo[k] + ((hi[k] - lo[k]) >> 1);
+            if (k < 3) {
+                lo[2 * k + 1] = lo[k];
+                hi[2 * k + 1] = mid - 1;
+                lo[2 * k + 2] = mid + 1;
+                hi[2 * k + 2] = hi[k];
+            }
+            const bool live = lo[k] <= hi[k];
+            const uint32_t j = live ? static_cast<uint32_t>(mid) : 0u;
+            const uint32_t i = live ? min(nsplit - j, lcm1) : 0u;
+            heavy[k] = j ? c.ld(c.prefix + j - 1) : 0.f;
+            light[k] = i ? c.ld(c.prefix + c.n - i) : 0.f;
+        }
+        int k = 0;
+#pragma unroll
+        for (int level = 0; level < 3; ++level) {
+            if (a > b) break;
+            float h = heavy[0], l = light[0];
+#pragma unroll
+            for (int q = 1; q < 7; ++q) {
+                h = k == q ? heavy[q] : h;
+                l = k == q ? light[q] : l;
+            }
+            const uint32_t j = static_cast<uint32_t>(a + ((b - a) >> 1));
+            bool le;
+            if constexpr (FF) {
+                const float d = __fsub_rn(__fadd_rn(h, l), tff.hi);
+                if (fabsf(d) > m) {
+                    le = d < 0.0f;
+                } else {
+                    const uint32_t i = min(nsplit - j, lcm1);
+                    const float hl = j ? c.ld(c.prefix_lo + j - 1) : 0.f;
+                    const float ll = i ? c.ld(c.prefix_lo + c.n - i) : 0.f;
+                    le = ff_sigma_minus(h, hl, l, ll, tff.hi, tff.lo) <= 0.0f;
+                }
+            } else {
+                le = __fadd_rn(l, h) <= target;
+            }
+            if (le)
+                a = static_cast<int>(j) + 1;
+            else
+                b = static_cast<int>(j) - 1;
+            k = 2 * k + (le ? 2 : 1);
+        }
+    }
+    split_at<R64, FF>(c, nsplit, target, tff, b, io, jo, spill);
 }
 
 // The top of the bisections of one CTA's splits, shared.  Every split of a CTA starts from
@@ -1511,35 +1681,39 @@ struct EntryStage {
     uint32_t h0, hcnt, l0, lcnt;
 };
 
-__device__ __forceinline__ float item_weight(const PackIn& c, uint32_t pos) {
-    if (c.elems) return __ldg(c.elems + pos);
-    const uint32_t widx = __ldg(c.idx + pos);
-    return widx < c.n ? __ldg(c.w + widx) : 0.f;
+template <class P>
+__device__ __forceinline__ float item_weight(const P& c, uint32_t pos) {
+    if (c.elems) return c.ld(c.elems + pos);
+    const uint32_t widx = c.ld(c.idx + pos);
+    return widx < c.n ? c.ld(c.w + widx) : 0.f;
 }
 
 // the entry of heavy position j packed with residual res (pack()'s heavy step)
-__device__ __forceinline__ void write_heavy(const PackIn& c, uint2* __restrict__ table,
+template <class P>
+__device__ __forceinline__ void write_heavy(const P& c, uint2* __restrict__ table,
                                             uint32_t j, float res, bool close_last) {
-    const uint32_t tidx = __ldg(c.idx + j);
+    const uint32_t tidx = c.ld(c.idx + j);
     const bool last = close_last && j + 1u == c.hc;
-    const uint32_t al = last ? tidx : __ldg(c.idx + j + 1u);
+    const uint32_t al = last ? tidx : c.ld(c.idx + j + 1u);
     const float p = last ? 1.0f : __fdiv_rn(res, c.mean);
     if (tidx < c.n) table[tidx] = make_uint2(__float_as_uint(p), al);
 }
 // the entry of light rank i packed while heavy position J was current (pack()'s light step)
-__device__ __forceinline__ void write_light(const PackIn& c, uint2* __restrict__ table,
+template <class P>
+__device__ __forceinline__ void write_light(const P& c, uint2* __restrict__ table,
                                             uint32_t i, uint32_t J) {
     const uint32_t pos = c.n - 1u - i;
-    const uint32_t tidx = __ldg(c.idx + pos);
-    const float weight = c.elems ? __ldg(c.elems + pos) : (tidx < c.n ? __ldg(c.w + tidx) : 0.f);
+    const uint32_t tidx = c.ld(c.idx + pos);
+    const float weight = c.elems ? c.ld(c.elems + pos) : (tidx < c.n ? c.ld(c.w + tidx) : 0.f);
     if (tidx < c.n)
-        table[tidx] = make_uint2(__float_as_uint(__fdiv_rn(weight, c.mean)), __ldg(c.idx + J));
+        table[tidx] = make_uint2(__float_as_uint(__fdiv_rn(weight, c.mean)), c.ld(c.idx + J));
 }
 
 // The walk's step is branch-free apart from the rare paths (ownership inside the look-ahead
 // window, positions outside the staged ranges): the weight is selected from the two
 // candidates, one 32-bit word is staged, and the stream that advanced loads its next weight.
-__device__ void pack_staged(const PackIn& c, const EntryStage& st, uint2* __restrict__ table,
+template <class P>
+__device__ void pack_staged(const P& c, const EntryStage& st, uint2* __restrict__ table,
                             uint32_t i0, uint32_t i1, uint32_t j0, uint32_t j1, float spill,
                             const LaterSplits* later) {
     uint32_t i = i0, j = j0;
@@ -1584,29 +1758,47 @@ __device__ void pack_staged(const PackIn& c, const EntryStage& st, uint2* __rest
 // i == i1.  Decisions, arithmetic and staged words are pack_staged's.  The successor of the stream
 // that advanced is loaded without a test: heavy position j + 1 <= heavyCount and light rank
 // i <= the light count are positions of the partition.
-template <bool ELEMS>
-__device__ __forceinline__ void pack_staged_fast(const PackIn& c, const EntryStage& st,
+//
+// Where the walks read from: the partition (ELEMS: its weights' own array), or a copy of the CTA's
+// weights in shared memory laid out like the staged words, with the successors of both ranges.
+enum class WalkFrom { kElems, kItems, kShared };
+template <WalkFrom FROM, class P>
+__device__ __forceinline__ void pack_staged_fast(const P& c, const EntryStage& st,
                                                  uint32_t i0, uint32_t i1, uint32_t j0,
-                                                 uint32_t j1, float spill) {
-    auto weight_at = [&](uint32_t pos) { return ELEMS ? __ldg(c.elems + pos) : item_weight(c, pos); };
+                                                 uint32_t j1, float spill,
+                                                 const float* shared = nullptr) {
     // staged word of heavy position j: st.w[j - h0]; of light rank i: st.w[q - h0], q = i + to_q
     const uint32_t to_q = st.h0 + st.hcnt - st.l0, q1 = i1 + to_q, light_pos = c.n - 1u + to_q;
     uint32_t* const w = st.w - st.h0;
+    auto weight_at = [&](uint32_t pos) {
+        return FROM == WalkFrom::kElems ? c.ld(c.elems + pos) : item_weight(c, pos);
+    };
+    // (shared: heavy positions up to h0 + hcnt + 1 at words [0, hcnt + 2), then the light ranks)
+    auto heavy_at = [&](uint32_t at) {
+        return FROM == WalkFrom::kShared ? shared[at - st.h0] : weight_at(at);
+    };
+    auto light_at = [&](uint32_t at) {
+        return FROM == WalkFrom::kShared ? shared[at - st.h0 + 2u] : weight_at(light_pos - at);
+    };
     uint32_t j = j0, q = i0 + to_q;
     if (j == j1 && q == q1) return;
     float wv = spill;
-    if (wv == 0.0f) wv = weight_at(j);
+    if (wv == 0.0f) wv = heavy_at(j);
     if (wv != wv) wv = __uint_as_float(0x7fffffffu);  // (a weight's NaN; sums' are this one)
     const uint32_t jmax = c.lcap == c.lc ? c.hc - 1u : c.hc;  // the current heavy's last position
-    float next_h = weight_at(j + 1u <= c.hc ? j + 1u : c.hc);
-    float next_l = weight_at(light_pos - q);
+    float next_h = heavy_at(j + 1u <= c.hc ? j + 1u : c.hc);
+    float next_l = light_at(q);
     do {
         const bool heavy_step = j != j1 && (q == q1 || wv <= c.mean);
         const float weight = heavy_step ? next_h : next_l;
         w[heavy_step ? j : q] = heavy_step ? __float_as_uint(wv) : min(j, jmax);
         j += heavy_step ? 1u : 0u;
         q += heavy_step ? 0u : 1u;
-        const float nw = weight_at(heavy_step ? min(j + 1u, c.hc) : light_pos - q);
+        float nw;
+        if constexpr (FROM == WalkFrom::kShared)
+            nw = shared[(heavy_step ? min(j + 1u, c.hc) : q + 2u) - st.h0];
+        else
+            nw = weight_at(heavy_step ? min(j + 1u, c.hc) : light_pos - q);
         next_h = heavy_step ? nw : next_h;
         next_l = heavy_step ? next_l : nw;
         wv = __fsub_rn(__fadd_rn(wv, weight), c.mean);
@@ -1672,6 +1864,186 @@ __global__ __launch_bounds__(kDescentThreads) void k_split_descent(SplitArgs a, 
     out[g] = st;
 }
 
+
+// One CTA's subproblems kb .. kb + npack: `k`, its split (si, sj) and residual per thread, the splits
+// of all slots (the look-ahead ones included) in s_i / s_j.  words: `stage` staged words of shared
+// memory; SHARED: the walks read the weights from a copy in shared memory (`weights`, stage + 3 words).
+template <uint32_t THREADS, uint32_t SLOTS, bool SHARED, class P>
+__device__ __forceinline__ void pack_cta(const P& c, uint2* table, uint32_t* status, uint32_t K,
+                                         uint32_t kb, uint32_t per_cta, uint32_t k, uint32_t si,
+                                         uint32_t sj, float spill, const uint32_t* s_i,
+                                         const uint32_t* s_j, uint32_t* words, uint32_t stage,
+                                         float* weights) {
+    // the CTA's heavy positions [s_j[0], s_j[npack]) and light ranks [s_i[0], s_i[npack]),
+    // with a margin for splits stepping back at the end; staged only if both fit
+    const uint32_t npack = min(per_cta, K - kb);
+    constexpr uint32_t kMargin = 64;
+    EntryStage es{words, s_j[0], 0u, s_i[0], 0u};
+    const uint32_t hspan = s_j[npack] > es.h0 ? s_j[npack] - es.h0 : 0u;
+    const uint32_t lspan = s_i[npack] > es.l0 ? s_i[npack] - es.l0 : 0u;
+    // the CTA's splits in slot order never step back (the common case): then no later
+    // subproblem covers an earlier one's items, and the ownership window is not consulted
+    const int slot1 = min(static_cast<int>(threadIdx.x) + 1, static_cast<int>(SLOTS) - 1);
+    const uint32_t i_next = s_i[slot1], j_next = s_j[slot1];
+    bool mono = i_next >= si && j_next >= sj;
+    if constexpr (SLOTS > THREADS) {
+        const uint32_t t2 = threadIdx.x + THREADS;
+        if (t2 + 1u < SLOTS) mono = mono && s_i[t2 + 1u] >= s_i[t2] && s_j[t2 + 1u] >= s_j[t2];
+    }
+    const bool all_mono = __syncthreads_and(mono);
+    auto walk = [&](uint32_t i0, uint32_t i1, uint32_t j0, uint32_t j1, float spill) {
+        if (c.elems)
+            pack_staged_fast<WalkFrom::kElems>(c, es, i0, i1, j0, j1, spill);
+        else
+            pack_staged_fast<WalkFrom::kItems>(c, es, i0, i1, j0, j1, spill);
+    };
+    // then, and within the heavy and light ranges, the CTA packs each position of [h0, h0 + hspan)
+    // and each rank of [l0, l0 + lspan) once: no word has to be marked, none to be tested
+    const bool exact = all_mono && s_j[npack] <= c.hc && s_i[npack] <= c.lc && hspan + lspan <= stage;
+    if (exact) {
+        es.hcnt = hspan;
+        es.lcnt = lspan;
+        if constexpr (SHARED) {
+            // the CTA's weights, with the successors of both ranges, for the walks
+            const uint32_t copied = hspan + lspan + 3u;
+            constexpr int kBatch = 8;  // loads in flight per thread
+            for (uint32_t q0 = threadIdx.x; q0 < copied; q0 += kBatch * THREADS) {
+                float v[kBatch];
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u) {
+                    const uint32_t q = min(q0 + u * THREADS, copied - 1u);
+                    v[u] = item_weight(c, q < hspan + 2u ? min(es.h0 + q, c.hc)
+                                                         : c.n - 1u - (es.l0 + q - hspan - 2u));
+                }
+#pragma unroll
+                for (int u = 0; u < kBatch; ++u)
+                    if (q0 + u * THREADS < copied) weights[q0 + u * THREADS] = v[u];
+            }
+            __syncthreads();
+            if (threadIdx.x < per_cta && k < K)
+                pack_staged_fast<WalkFrom::kShared>(c, es, si, i_next, sj, j_next, spill, weights);
+        } else {
+            if (threadIdx.x < per_cta && k < K) walk(si, i_next, sj, j_next, spill);
+        }
+    } else {
+        // with a margin for splits stepping back at the end; staged only if both fit
+        if (hspan + lspan + 2u * kMargin <= stage) {
+            es.hcnt = hspan + kMargin;
+            es.lcnt = lspan + kMargin;
+        }
+        for (uint32_t q = threadIdx.x; q < es.hcnt + es.lcnt; q += THREADS)
+            es.w[q] = kNotStaged;
+        __syncthreads();
+        const int t = threadIdx.x;
+        if (threadIdx.x < per_cta && k < K) {
+            const uint32_t i1 = max(i_next, si), j1 = max(j_next, sj);
+            bool clean = true;
+            int count = 0;
+            if (!all_mono) {
+                count = static_cast<int>(min(static_cast<uint32_t>(kSplitLook), K - 1u - k));
+                for (int d = 1; d <= count; ++d)
+                    clean = clean && s_i[t + d] >= i1 && s_j[t + d] >= j1;
+                if (k + kSplitLook + 1u < K &&
+                    (s_i[t + kSplitLook + 1] < i1 || s_j[t + kSplitLook + 1] < j1))
+                    atomicOr(status, kStatusNonMonotone);
+            }
+            const LaterSplits later{s_i, s_j, t, count};
+            const bool inside = sj >= es.h0 && j1 - es.h0 <= es.hcnt && si >= es.l0 &&
+                                i1 - es.l0 <= es.lcnt && j1 <= c.hc && i1 <= c.lc;
+            if (clean && inside)
+                walk(si, i1, sj, j1, spill);
+            else
+                pack_staged(c, es, table, si, i1, sj, j1, spill, clean ? nullptr : &later);
+        }
+    }
+    __syncthreads();
+    // write-out: consecutive lanes on consecutive positions, kOutBatch positions per thread
+    // with their loads in flight together (write_heavy / write_light's values; positions
+    // clamped into [0, n) so that every load is in bounds, only staged entries stored)
+    const bool close_last = c.lcap == c.lc;
+    constexpr int kOutBatch = SHARED ? 6 : 3;  // (2 and 4: 442 us where 3 takes 415, uniform n = 2^26)
+    const uint32_t bd = THREADS, nm1 = c.n - 1u;
+    if (exact && c.elems && !(close_last && es.h0 + es.hcnt == c.hc)) {
+        // every word is staged, every position and its successor lie in the partition
+        const uint32_t* const hidx = c.idx + es.h0;
+        for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
+            uint32_t t[kOutBatch], al[kOutBatch];
+            float r[kOutBatch];
+#pragma unroll
+            for (int u = 0; u < kOutBatch; ++u) {
+                const uint32_t q = q0 + u * bd;
+                t[u] = c.n;
+                if (q < es.hcnt) {
+                    r[u] = __uint_as_float(es.w[q]);
+                    t[u] = c.ld(hidx + q);
+                    al[u] = c.ld(hidx + q + 1u);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kOutBatch; ++u)
+                if (t[u] < c.n)
+                    table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(r[u], c.mean)), al[u]);
+        }
+        const uint32_t* const lidx = c.idx + (nm1 - es.l0);
+        const float* const lelem = c.elems + (nm1 - es.l0);
+        const uint32_t* const lw = es.w + es.hcnt;
+        for (uint32_t q0 = threadIdx.x; q0 < es.lcnt; q0 += kOutBatch * bd) {
+            uint32_t t[kOutBatch], aj[kOutBatch];
+            float wt[kOutBatch];
+#pragma unroll
+            for (int u = 0; u < kOutBatch; ++u) {
+                const uint32_t q = q0 + u * bd;
+                t[u] = c.n;
+                if (q < es.lcnt) {
+                    t[u] = c.ld(lidx - q);
+                    wt[u] = c.ld(lelem - q);
+                    aj[u] = c.ld(c.idx + lw[q]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < kOutBatch; ++u)
+                if (t[u] < c.n)
+                    table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(wt[u], c.mean)), aj[u]);
+        }
+        return;
+    }
+    for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
+        uint32_t r[kOutBatch], t[kOutBatch], al[kOutBatch];
+#pragma unroll
+        for (int u = 0; u < kOutBatch; ++u) {
+            const uint32_t q = q0 + u * bd;
+            r[u] = q < es.hcnt ? es.w[q] : kNotStaged;
+            const uint32_t j = min(es.h0 + q, nm1);
+            t[u] = c.ld(c.idx + j);
+            al[u] = c.ld(c.idx + min(j + 1u, nm1));
+        }
+#pragma unroll
+        for (int u = 0; u < kOutBatch; ++u) {
+            if (r[u] == kNotStaged || t[u] >= c.n) continue;
+            const bool last = close_last && es.h0 + q0 + u * bd + 1u == c.hc;
+            const float p = last ? 1.0f : __fdiv_rn(__uint_as_float(r[u]), c.mean);
+            table[t[u]] = make_uint2(__float_as_uint(p), last ? t[u] : al[u]);
+        }
+    }
+    for (uint32_t q0 = threadIdx.x; q0 < es.lcnt; q0 += kOutBatch * bd) {
+        uint32_t J[kOutBatch], t[kOutBatch], aj[kOutBatch];
+        float wt[kOutBatch];
+#pragma unroll
+        for (int u = 0; u < kOutBatch; ++u) {
+            const uint32_t q = q0 + u * bd;
+            J[u] = q < es.lcnt ? es.w[es.hcnt + q] : kNotStaged;
+            const uint32_t pos = nm1 - min(es.l0 + q, nm1);
+            t[u] = c.ld(c.idx + pos);
+            wt[u] = c.elems ? c.ld(c.elems + pos) : (t[u] < c.n ? c.ld(c.w + t[u]) : 0.f);
+            aj[u] = c.ld(c.idx + min(J[u], nm1));
+        }
+#pragma unroll
+        for (int u = 0; u < kOutBatch; ++u) {
+            if (J[u] == kNotStaged || t[u] >= c.n) continue;
+            table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(wt[u], c.mean)), aj[u]);
+        }
+    }
+}
 
 // Bound by instruction issue (60 % active) and the L1's wavefronts (69 %) together; 146 instructions
 // per weight in the float-float form, where it took 224.  n = 2^26, split size 12: 0.500 -> 0.415 ms
@@ -1768,154 +2140,10 @@ __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, Ba
     // there; the inline kernel's bisections lose more to the smaller L1 than its walks gain)
     extern __shared__ uint2 s_items[];
     if constexpr (!RECORDS) {
-        // the CTA's heavy positions [s_j[0], s_j[npack]) and light ranks [s_i[0], s_i[npack]),
-        // with a margin for splits stepping back at the end; staged only if both fit
-        const uint32_t kb = blk * kSplitPack;
-        const uint32_t npack = min(static_cast<uint32_t>(kSplitPack), K - kb);
-        constexpr uint32_t kMargin = 64;
-        EntryStage es{reinterpret_cast<uint32_t*>(s_items), s_j[0], 0u, s_i[0], 0u};
-        const uint32_t stage = stage_entries_for(a.split_size);
-        const uint32_t hspan = s_j[npack] > es.h0 ? s_j[npack] - es.h0 : 0u;
-        const uint32_t lspan = s_i[npack] > es.l0 ? s_i[npack] - es.l0 : 0u;
-        // the CTA's splits in slot order never step back (the common case): then no later
-        // subproblem covers an earlier one's items, and the ownership window is not consulted
-        const int slot1 = min(static_cast<int>(threadIdx.x) + 1, kSplitSlots - 1);
-        const uint32_t i_next = s_i[slot1], j_next = s_j[slot1];
-        const bool all_mono = __syncthreads_and(i_next >= si[0] && j_next >= sj[0]);
-        auto walk = [&](uint32_t i0, uint32_t i1, uint32_t j0, uint32_t j1, float spill) {
-            if (c.elems)
-                pack_staged_fast<true>(c, es, i0, i1, j0, j1, spill);
-            else
-                pack_staged_fast<false>(c, es, i0, i1, j0, j1, spill);
-        };
-        // then, and within the heavy and light ranges, the CTA packs each position of [h0, h0 + hspan)
-        // and each rank of [l0, l0 + lspan) once: no word has to be marked, none to be tested
-        const bool exact = all_mono && s_j[npack] <= c.hc && s_i[npack] <= c.lc && hspan + lspan <= stage;
-        if (exact) {
-            es.hcnt = hspan;
-            es.lcnt = lspan;
-            if (threadIdx.x < kSplitPack && kv[0] < K) walk(si[0], i_next, sj[0], j_next, sp[0]);
-        } else {
-            // with a margin for splits stepping back at the end; staged only if both fit
-            if (hspan + lspan + 2u * kMargin <= stage) {
-                es.hcnt = hspan + kMargin;
-                es.lcnt = lspan + kMargin;
-            }
-            for (uint32_t q = threadIdx.x; q < es.hcnt + es.lcnt; q += blockDim.x)
-                es.w[q] = kNotStaged;
-            __syncthreads();
-#pragma unroll 1
-            for (int v = 0; v < kSplitPerThread; ++v) {
-                const int t = threadIdx.x + v * kSplitThreads;
-                const uint32_t k = kv[v];
-                if (t >= kSplitPack || k >= K) continue;
-                const uint32_t i1 = max(s_i[t + 1], si[v]), j1 = max(s_j[t + 1], sj[v]);
-                bool clean = true;
-                int count = 0;
-                if (!all_mono) {
-                    count = static_cast<int>(min(static_cast<uint32_t>(kSplitLook), K - 1u - k));
-                    for (int d = 1; d <= count; ++d)
-                        clean = clean && s_i[t + d] >= i1 && s_j[t + d] >= j1;
-                    if (k + kSplitLook + 1u < K &&
-                        (s_i[t + kSplitLook + 1] < i1 || s_j[t + kSplitLook + 1] < j1))
-                        atomicOr(a.status, kStatusNonMonotone);
-                }
-                const LaterSplits later{s_i, s_j, t, count};
-                const bool inside = sj[v] >= es.h0 && j1 - es.h0 <= es.hcnt && si[v] >= es.l0 &&
-                                    i1 - es.l0 <= es.lcnt && j1 <= c.hc && i1 <= c.lc;
-                if (clean && inside)
-                    walk(si[v], i1, sj[v], j1, sp[v]);
-                else
-                    pack_staged(c, es, table, si[v], i1, sj[v], j1, sp[v], clean ? nullptr : &later);
-            }
-        }
-        __syncthreads();
-        // write-out: consecutive lanes on consecutive positions, kOutBatch positions per thread
-        // with their loads in flight together (write_heavy / write_light's values; positions
-        // clamped into [0, n) so that every load is in bounds, only staged entries stored)
-        const bool close_last = c.lcap == c.lc;
-        constexpr int kOutBatch = 3;  // (2 and 4: 442 us where 3 takes 415, uniform n = 2^26)
-        const uint32_t bd = kSplitThreads, nm1 = c.n - 1u;
-        if (exact && c.elems && !(close_last && es.h0 + es.hcnt == c.hc)) {
-            // every word is staged, every position and its successor lie in the partition
-            const uint32_t* const hidx = c.idx + es.h0;
-            for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
-                uint32_t t[kOutBatch], al[kOutBatch];
-                float r[kOutBatch];
-#pragma unroll
-                for (int u = 0; u < kOutBatch; ++u) {
-                    const uint32_t q = q0 + u * bd;
-                    t[u] = c.n;
-                    if (q < es.hcnt) {
-                        r[u] = __uint_as_float(es.w[q]);
-                        t[u] = __ldg(hidx + q);
-                        al[u] = __ldg(hidx + q + 1u);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kOutBatch; ++u)
-                    if (t[u] < c.n)
-                        table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(r[u], c.mean)), al[u]);
-            }
-            const uint32_t* const lidx = c.idx + (nm1 - es.l0);
-            const float* const lelem = c.elems + (nm1 - es.l0);
-            const uint32_t* const lw = es.w + es.hcnt;
-            for (uint32_t q0 = threadIdx.x; q0 < es.lcnt; q0 += kOutBatch * bd) {
-                uint32_t t[kOutBatch], aj[kOutBatch];
-                float wt[kOutBatch];
-#pragma unroll
-                for (int u = 0; u < kOutBatch; ++u) {
-                    const uint32_t q = q0 + u * bd;
-                    t[u] = c.n;
-                    if (q < es.lcnt) {
-                        t[u] = __ldg(lidx - q);
-                        wt[u] = __ldg(lelem - q);
-                        aj[u] = __ldg(c.idx + lw[q]);
-                    }
-                }
-#pragma unroll
-                for (int u = 0; u < kOutBatch; ++u)
-                    if (t[u] < c.n)
-                        table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(wt[u], c.mean)), aj[u]);
-            }
-            return;
-        }
-        for (uint32_t q0 = threadIdx.x; q0 < es.hcnt; q0 += kOutBatch * bd) {
-            uint32_t r[kOutBatch], t[kOutBatch], al[kOutBatch];
-#pragma unroll
-            for (int u = 0; u < kOutBatch; ++u) {
-                const uint32_t q = q0 + u * bd;
-                r[u] = q < es.hcnt ? es.w[q] : kNotStaged;
-                const uint32_t j = min(es.h0 + q, nm1);
-                t[u] = __ldg(c.idx + j);
-                al[u] = __ldg(c.idx + min(j + 1u, nm1));
-            }
-#pragma unroll
-            for (int u = 0; u < kOutBatch; ++u) {
-                if (r[u] == kNotStaged || t[u] >= c.n) continue;
-                const bool last = close_last && es.h0 + q0 + u * bd + 1u == c.hc;
-                const float p = last ? 1.0f : __fdiv_rn(__uint_as_float(r[u]), c.mean);
-                table[t[u]] = make_uint2(__float_as_uint(p), last ? t[u] : al[u]);
-            }
-        }
-        for (uint32_t q0 = threadIdx.x; q0 < es.lcnt; q0 += kOutBatch * bd) {
-            uint32_t J[kOutBatch], t[kOutBatch], aj[kOutBatch];
-            float wt[kOutBatch];
-#pragma unroll
-            for (int u = 0; u < kOutBatch; ++u) {
-                const uint32_t q = q0 + u * bd;
-                J[u] = q < es.lcnt ? es.w[es.hcnt + q] : kNotStaged;
-                const uint32_t pos = nm1 - min(es.l0 + q, nm1);
-                t[u] = __ldg(c.idx + pos);
-                wt[u] = c.elems ? __ldg(c.elems + pos) : (t[u] < c.n ? __ldg(c.w + t[u]) : 0.f);
-                aj[u] = __ldg(c.idx + min(J[u], nm1));
-            }
-#pragma unroll
-            for (int u = 0; u < kOutBatch; ++u) {
-                if (J[u] == kNotStaged || t[u] >= c.n) continue;
-                table[t[u]] = make_uint2(__float_as_uint(__fdiv_rn(wt[u], c.mean)), aj[u]);
-            }
-        }
+        pack_cta<kSplitThreads, kSplitSlots, false>(
+            c, table, a.status, K, blk * kSplitPack, static_cast<uint32_t>(kSplitPack), kv[0],
+            si[0], sj[0], sp[0], s_i, s_j, reinterpret_cast<uint32_t*>(s_items),
+            stage_entries_for(a.split_size), nullptr);
         return;
     }
     PackWin win{s_items, 0u, 0u, 0u, 0u};
@@ -1951,6 +2179,166 @@ __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, Ba
         const LaterSplits later{s_i, s_j, t, count};
         pack(c, win, table, si[v], i1, sj[v], j1, sp[v], clean ? nullptr : &later);
     }
+}
+
+// ---------------------------------------------------------------------------------
+// one small distribution: total mass, partition and split-pack in one launch
+// ---------------------------------------------------------------------------------
+
+// A cluster of at most 8 CTAs (the portable size), the first of which hold a tile each.  Three
+// dependent launches of a few microseconds each -- their starts, the total's and the lookback's trips
+// through L2, the weights read twice -- are what a small build costs; here the tile stays parked in
+// shared memory between the phases, the tiles' masses and aggregates go straight into the other CTAs'
+// shared memory, and cluster barriers order the phases.  The results are those of k_total_mass,
+// k_prefix_partition and k_split_pack, whose pieces do the work (the same sums in the same order; the
+// carries are exact, or added tile by tile in FP32 mode).  The subproblems are shared out evenly; every
+// load waits alone here, so bisections read three levels at a time and the walks' weights come through
+// shared memory.  Builds one after the other, three launches -> this one: n = 1000, split size 2, FP32
+// 12.2 -> 9.0 us; n = 4096, 12, float-float 18.2 -> 14.8; n = 16384, 12, float-float 23.0 -> 17.4; n =
+// 32768, 32, float-float 48 -> 22.  At n = 1000 the load and the mass take 2 us of it, mean and
+// partition 3.4, splits 1.8, walks and write-out 1.9.
+constexpr uint32_t kSmallCtas = 8;
+constexpr uint32_t kSmallPack = kTileThreads;  // subproblems per CTA, at most: one per thread
+constexpr uint32_t kSmallSlots = kSmallPack + kSplitLook + 1;
+constexpr uint32_t kSmallStage = kPartBytes / 8u - 4u;  // staged words; as many weights and 3 more
+
+template <bool R64, bool COMP, bool FFOUT>
+__global__ __launch_bounds__(kTileThreads, 1) void k_build_small(PartArgs a, SplitArgs sa) {
+    pdl_entry();
+    cluster_arrive();
+    __shared__ __align__(16) unsigned char s_raw[kPartBytes];
+    __shared__ ff s_part[kTileWarps];
+    __shared__ double s_mass[kSmallCtas];
+    __shared__ PartAgg s_agg[kSmallCtas];
+    __shared__ uint32_t s_hc;
+    __shared__ double s_total;
+    __shared__ float2 s_mean;
+    __shared__ uint32_t s_i[kSmallSlots], s_j[kSmallSlots];
+    const uint32_t rank = blockIdx.x, ctas = gridDim.x, n = a.n, tiles = tiles_for(n);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    if (rank < tiles) {
+        float x[4][4];
+        load_tile(a.w, n, rank, x);
+        float4* const s_x = reinterpret_cast<float4*>(s_raw);
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+            s_x[park_slot(warp * 128 + v * 32 + lane)] = make_float4(x[v][0], x[v][1], x[v][2], x[v][3]);
+        tile_mass_warp(x, s_part);
+    }
+    __syncthreads();
+    cluster_wait();  // every CTA of the cluster runs: its shared memory may be written
+    if (rank < tiles && warp == 0) {
+        const double mass = tile_mass(s_part);
+        if (static_cast<uint32_t>(lane) < ctas) st_cluster(s_mass + rank, lane, mass);
+    }
+    cluster_arrive();
+    cluster_wait();
+    // the sum of k_total_mass's last CTA: its tree over 32 lanes, where the others add zeros
+    if (warp == 0) {
+        double t = 0.0;
+        if (static_cast<uint32_t>(lane) < tiles) t = __dadd_rn(t, s_mass[lane]);
+        if (tiles > 1u) {
+#pragma unroll
+            for (int m = 4; m > 0; m >>= 1) t = __dadd_rn(t, __shfl_xor_sync(0xffffffffu, t, m));
+        }
+        if (lane == 0) {
+            const Mean m = mean_of(t, n);
+            s_total = t;
+            s_mean = make_float2(m.hi, m.lo);
+            if (rank == 0) {
+                a.ctrl->total = t;
+                a.ctrl->mean64 = m.m64;
+                a.ctrl->mean = m.hi;
+                a.ctrl->mean_lo = m.lo;
+                a.ctrl->block_reads = 0ull;
+            }
+        }
+    }
+    __syncthreads();
+    const float mean = s_mean.x, mean_lo = s_mean.y;
+    if (rank < tiles) {
+        partition_tile<COMP, FFOUT, false, Carry::kCluster>(
+            a, BatchView{}, s_raw, ClusterPart{rank, tiles, ctas, s_total, mean, s_agg, &s_hc});
+    } else {
+        cluster_arrive();  // partition_tile's
+        cluster_wait();
+        if (threadIdx.x == 0) {
+            uint32_t hc = 0;
+            for (uint32_t r = 0; r < tiles; ++r) hc += s_agg[r].c;
+            s_hc = hc;
+        }
+    }
+    // (orders the cluster's partition before the loads below, and this CTA's s_hc)
+    cluster_arrive();
+    cluster_wait();
+    const uint32_t hc = s_hc;
+    if (hc == 0u || hc >= n) {
+        for (uint32_t e = rank * kTileThreads + threadIdx.x; e < n; e += ctas * kTileThreads)
+            sa.table[e] = make_uint2(__float_as_uint(1.0f), e);
+        return;
+    }
+    const PackOwn c{PackIn{a.w, a.idx, a.elems, a.prefix, a.prefix_lo, n, hc, n - hc,
+                           sa.full_light ? n - hc : n - hc - 1u, mean, mean_lo}};
+    const uint32_t K = splits_for(n, sa.split_size);
+    const uint32_t per = (K + ctas - 1u) / ctas, kb = rank * per;
+    if (kb >= K) return;
+    uint32_t si = 0, sj = 0;
+    float sp = 0.f;
+#pragma unroll 1
+    for (uint32_t slot = threadIdx.x; slot < kSmallSlots; slot += kTileThreads) {
+        const uint32_t k = kb + slot;
+        const bool on = k != 0u && k < K && slot < per + kSplitLook + 1u;
+        uint32_t i = k == 0u ? 0u : c.lc, j = k == 0u ? 0u : hc;
+        float r = 0.f;
+        bisect_wide<R64, FFOUT>(c, on ? k * sa.split_size : 0u, on, i, j, r);
+        s_i[slot] = i;
+        s_j[slot] = j;
+        if (slot == threadIdx.x) {
+            si = i;
+            sj = j;
+            sp = r;
+        }
+    }
+    __syncthreads();
+    uint32_t* const words = reinterpret_cast<uint32_t*>(s_raw);
+    pack_cta<kTileThreads, kSmallSlots, true>(c, sa.table, sa.status, K, kb, per, kb + threadIdx.x,
+                                              si, sj, sp, s_i, s_j, words, kSmallStage,
+                                              reinterpret_cast<float*>(words + kSmallStage));
+}
+
+// CTAs of the cluster: a tile each, and no thread with two splits if 8 CTAs can avoid it
+static uint32_t small_ctas(uint32_t n, uint32_t split_size) {
+    constexpr uint32_t one_each = kSmallPack - kSplitLook - 1u;
+    const uint32_t split = (splits_for(n, split_size) + one_each - 1u) / one_each;
+    return split > kSmallCtas ? kSmallCtas : (split > tiles_for(n) ? split : tiles_for(n));
+}
+
+bool small_build(uint32_t n, uint32_t split_size) {
+    return tiles_for(n) <= kSmallCtas && splits_for(n, split_size) <= kSmallCtas * kSmallPack;
+}
+
+cudaError_t launch_build_small(cudaStream_t st, bool comp, bool r64, bool full_light,
+                               const float* w, uint32_t n, BuildCtrl* ctrl, uint32_t* idx,
+                               float* prefix, float* elems, float* prefix_lo, uint32_t split_size,
+                               uint2* table) {
+    PartArgs a{};
+    a.w = w;
+    a.n = n;
+    a.ctrl = ctrl;
+    a.idx = idx;
+    a.prefix = prefix;
+    a.elems = elems;
+    a.prefix_lo = prefix_lo;
+    SplitArgs sa{};
+    sa.table = table;
+    sa.status = &ctrl->status;
+    sa.split_size = split_size;
+    sa.full_light = full_light ? 1u : 0u;
+    auto kernel = prefix_lo ? k_build_small<true, true, true>
+                  : comp    ? (r64 ? k_build_small<true, true, false> : k_build_small<false, true, false>)
+                            : (r64 ? k_build_small<true, false, false> : k_build_small<false, false, false>);
+    const uint32_t ctas = small_ctas(n, split_size);
+    return launch_cluster(ctas, kernel, ctas, kTileThreads, st, a, sa);
 }
 
 // the staging window is dynamic shared memory above the 48 KB static limit

@@ -588,6 +588,13 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
     float* lo = float_float(h) ? b->prefix_lo : nullptr;
     b->blocks_n = 0;
     const bool blocks = b->blocks && n > kBlockMinN && n <= kBlockMaxN;
+    if (h->cfg.split_pack_mode == WRS_SPLITPACK_INLINE && small_build(n, h->cfg.split_size)) {
+        WRS_CUDA(launch_build_small(st, comp, h->cfg.split_residual_f64 != 0,
+                                    h->cfg.split_full_light != 0, weights, n, b->ctrl, b->idx,
+                                    b->prefix, elems, lo, h->cfg.split_size, b->table),
+                 "small build");
+        return WRS_OK;
+    }
     WRS_CUDA(launch_total_mass(st, weights, n, b->partials, b->ctrl), "total mass");
     WRS_CUDA(launch_prefix_partition(st, comp, weights, n, b->ctrl, b->part_states, b->cap_tiles,
                                      b->idx, b->prefix, elems, lo,

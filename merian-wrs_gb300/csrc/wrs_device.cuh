@@ -41,6 +41,29 @@ __device__ __forceinline__ void pdl_entry() {
     if (gridDim.x <= kPdlMaxGrid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// Thread-block clusters.  arrive releases this thread's writes to the cluster's CTAs (shared and
+// global memory), wait acquires theirs; every thread of the cluster does both, in turn.
+__device__ __forceinline__ void cluster_arrive() {
+    __syncwarp();  // (.aligned: a warp's threads arrive together)
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// *p = v in the shared memory of the cluster's CTA `rank` (p: the variable in this CTA's)
+template <class T>
+__device__ __forceinline__ void st_cluster(T* p, uint32_t rank, const T& v) {
+    static_assert(sizeof(T) % 4 == 0, "whole words");
+    uint32_t at, words[sizeof(T) / 4];
+    __builtin_memcpy(words, &v, sizeof(T));
+    asm("mapa.shared::cluster.u32 %0, %1, %2;"
+        : "=r"(at)
+        : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(p))), "r"(rank));
+#pragma unroll
+    for (uint32_t i = 0; i < sizeof(T) / 4; ++i)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(at + 4u * i), "r"(words[i]) : "memory");
+}
+
 // ---------------------------------------------------------------------------
 // float-float arithmetic (Knuth two-sum); every operation rounds once.
 // ---------------------------------------------------------------------------

@@ -144,10 +144,35 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
                               cudaStream_t st, Args&&... args) {
     return launch_overlapped(true, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
+// launch_pdl with clusters of `cluster` CTAs (at most 8)
+template <class... KArgs, class... Args>
+inline cudaError_t launch_cluster(uint32_t cluster, void (*kernel)(KArgs...), dim3 grid, dim3 block,
+                                  cudaStream_t st, Args&&... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = cluster;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 2;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
+}
 
 // ---- launchers (defined in wrs_build.cu / wrs_sample.cu) -------------------------
 cudaError_t launch_total_mass(cudaStream_t st, const float* w, uint32_t n, double* partials,
                               BuildCtrl* ctrl);
+// total mass, partition and split-pack in one launch, for the sizes small_build() names
+bool small_build(uint32_t n, uint32_t split_size);
+cudaError_t launch_build_small(cudaStream_t st, bool comp, bool r64, bool full_light,
+                               const float* w, uint32_t n, BuildCtrl* ctrl, uint32_t* idx,
+                               float* prefix, float* elems, float* prefix_lo, uint32_t split_size,
+                               uint2* table);
 cudaError_t launch_prefix_partition(cudaStream_t st, bool comp, const float* w, uint32_t n,
                                     BuildCtrl* ctrl, PartState* states, uint32_t cap_tiles,
                                     uint32_t* idx_out, float* prefix_out, float* elems_out,
