@@ -59,7 +59,7 @@ struct wrs_buffers {
     AliasBlock* blocks = nullptr;  // alias: the table's alias blocks (kBlockMinN < n)
     uint32_t* classes = nullptr;   // the partition's heavy bits, for the blocks
     uint32_t blocks_n = 0;         // the n the last build wrote the alias blocks for (0: none)
-    uint32_t* coarse = nullptr;  // scratch of the guiding-table / cell construction
+    uint32_t* group = nullptr;  // scratch of the guiding-table / cell construction
     uint32_t* tile_scratch = nullptr;  // block-wise baselines: 3 words per tile
     int2* descent = nullptr;           // split-pack: shared bisection tops per CTA
 };
@@ -90,7 +90,7 @@ size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 
 struct Layout {
     size_t ctrl, partials, part_states, scan_states, idx, prefix, elems, prefix_lo, table, records,
-        blocks, classes, cmf, guide, cells, tree, coarse, tile_scratch, descent, total;
+        blocks, classes, cmf, guide, cells, tree, group, tile_scratch, descent, total;
 };
 
 // ITS bisects the whole CMF with the non-cooperative sampler, and its CMF is deep enough for
@@ -150,7 +150,7 @@ Layout layout_for(const wrs_config& cfg, uint32_t max_n) {
         else if (G)
             L.cells = take(sizeof(ItsCell) * G);  // (the grid has fewer cells, of the same size)
         if (G && (its || cfg.scan_precision != WRS_SCAN_FP32))
-            L.coarse = take(sizeof(uint32_t) * (coarse_entries(G) + group_entries(G)));
+            L.group = take(sizeof(uint32_t) * group_entries(G));
         // ITS bisecting the whole CMF (FP32, or no cells): the probe tree's deeper levels
         if (its_tree_levels(cfg, max_n))
             L.tree = take(sizeof(TreeBlock) * its_tree_blocks(its_tree_stored_levels(max_n)));
@@ -295,7 +295,7 @@ wrs_status wrs_buffers_create(const wrs_handle* h, uint32_t max_n, wrs_buffers**
         b->guide = L.guide ? reinterpret_cast<uint32_t*>(p + L.guide) : nullptr;
         b->cells = L.cells ? reinterpret_cast<ItsCell*>(p + L.cells) : nullptr;
         b->tree = L.tree ? reinterpret_cast<TreeBlock*>(p + L.tree) : nullptr;
-        b->coarse = L.coarse ? reinterpret_cast<uint32_t*>(p + L.coarse) : nullptr;
+        b->group = L.group ? reinterpret_cast<uint32_t*>(p + L.group) : nullptr;
     }
     e = cudaMemset(b->base, 0, zeroed_bytes(h->cfg, max_n));
     if (e == cudaSuccess) e = cudaDeviceSynchronize();
@@ -359,8 +359,8 @@ static wrs_status check_tables(const wrs_handle* h, const wrs_buffers* b) {
     if ((h->cfg.method == WRS_METHOD_CUTPOINT || its_guided(h)) &&
         b->cfg.guiding_entry_size != h->cfg.guiding_entry_size)
         return fail(WRS_ERR_INVALID_ARG, "buffers were created for another guiding_entry_size");
-    if ((its_guided(h) && (!b->cells || !b->coarse)) ||
-        (h->cfg.method == WRS_METHOD_CUTPOINT && compensated(h) && !b->coarse))
+    if ((its_guided(h) && (!b->cells || !b->group)) ||
+        (h->cfg.method == WRS_METHOD_CUTPOINT && compensated(h) && !b->group))
         return fail(WRS_ERR_INVALID_ARG,
                     "buffers were created without the cell blocks or the construction scratch "
                     "this handle's search uses");
@@ -552,7 +552,7 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
         const uint32_t G = guide_entries(n, h->cfg.guiding_entry_size);
         if (comp) b->monotone_n = n;
         if (h->cfg.method == WRS_METHOD_CUTPOINT)
-            WRS_CUDA(comp ? launch_guide_monotone(st, b->cmf, n, G, b->coarse, b->guide)
+            WRS_CUDA(comp ? launch_guide_monotone(st, b->cmf, n, G, b->group, b->guide)
                           : launch_cutpoint_guide(st, b->cmf, n, G, b->guide),
                      "guiding table");
         else if (its_guided(h)) {
@@ -560,11 +560,11 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
             b->cells_grid = comp;
             if (comp) {
                 WRS_CUDA(launch_its_grids(st, b->cmf, n, its_grids(n, h->cfg.guiding_entry_size),
-                                          b->coarse, reinterpret_cast<ItsGrid*>(b->cells)),
+                                          b->group, reinterpret_cast<ItsGrid*>(b->cells)),
                          "ITS grid");
             } else {
                 // an FP32 CMF need not be monotone: mark the cells the search cannot serve
-                WRS_CUDA(launch_its_cells(st, b->cmf, n, G, b->coarse, b->cells), "ITS cells");
+                WRS_CUDA(launch_its_cells(st, b->cmf, n, G, b->group, b->cells), "ITS cells");
                 WRS_CUDA(launch_its_marks(st, b->cmf, n, G, b->cells,
                                           reinterpret_cast<float*>(b->tile_scratch),
                                           b->tile_scratch + 2u * b->cap_tiles),

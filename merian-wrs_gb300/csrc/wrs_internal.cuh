@@ -317,17 +317,11 @@ cudaError_t launch_its_sample(cudaStream_t st, uint32_t rng, uint32_t coop, bool
 
 cudaError_t launch_cutpoint_guide(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                   uint32_t* guide);
-// the same table for an exactly non-decreasing CMF (galloping searches)
-// (coarse: scratch of coarse_entries(G) + group_entries(G) words: every kCoarseStride-th
-// entry, then every 32nd, bracketing the searches of the others)
-constexpr uint32_t kCoarseStride = 1024;
-__host__ __device__ inline uint32_t coarse_entries(uint32_t G) {
-    return (G + kCoarseStride - 1) / kCoarseStride + 1;
-}
-// starts of the groups of 32 cells (the third pass's brackets), after the coarse ones
+// the same table for an exactly non-decreasing CMF (group: scratch of group_entries(G) words, every
+// 32nd entry, bracketing the searches of the others)
 __host__ __device__ inline uint32_t group_entries(uint32_t G) { return (G + 31u) / 32u + 1u; }
 cudaError_t launch_guide_monotone(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                                  uint32_t* coarse, uint32_t* guide);
+                                  uint32_t* group, uint32_t* guide);
 // ITS on the FP32 CMF through cells: cell k of G equal-mass cells (the Cutpoint guiding table's) =
 // its candidate range [x, y] and the CMF at the last index of each of the range's kCellParts parts
 // of d = ceil((y - x + 1) / kCellParts) indices; one 32-byte sector
@@ -338,7 +332,7 @@ struct alignas(32) ItsCell {
 };
 static_assert(sizeof(ItsCell) == 32, "one cell block is one 32-byte sector");
 cudaError_t launch_its_cells(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsCell* cells);
+                             uint32_t* group, ItsCell* cells);
 cudaError_t launch_its_sample_cells(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
                                     const ItsCell* cells, uint32_t G, uint64_t S, uint64_t seed,
                                     uint64_t offset, uint32_t* out, const TreeBlock* blocks,
@@ -368,7 +362,7 @@ __host__ __device__ inline uint32_t its_grids(uint32_t n, uint32_t entry) {
     return static_cast<uint32_t>(g < (1u << 24) ? g : (1u << 24));
 }
 cudaError_t launch_its_grids(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsGrid* grids);
+                             uint32_t* group, ItsGrid* grids);
 cudaError_t launch_its_sample_grids(cudaStream_t st, uint32_t rng, const float* cmf, uint32_t n,
                                     const ItsGrid* grids, uint32_t G, uint64_t S, uint64_t seed,
                                     uint64_t offset, uint32_t* out);

@@ -712,9 +712,8 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_tree(const float*
 // Results equal the bisection's (k_its_sample_tree's).
 
 // Starts x_k = lower bound of c_k = fl(step * k) (clamped to N - 1) of the equal-mass cells of
-// a non-decreasing CMF, in three passes, each bracketing the next (c_k is non-decreasing in k,
-// so x_k is too).  k_cell_coarse bisects the whole CMF for every kCoarseStride-th start;
-// k_cell_groups bisects, inside those brackets, for the first start of every group of 32
+// a non-decreasing CMF, in two passes, the first bracketing the second (c_k is non-decreasing in k,
+// so x_k is too).  k_cell_groups bisects the whole CMF for the first start of every group of 32
 // cells; then one warp per group finds its 32 starts in the group's bracket [x_{32g},
 // x_{32(g+1)}]: where that holds at most 128 values, the lanes load them with one coalesced
 // pass and each start is the bracket's start plus the number of values below its threshold,
@@ -750,40 +749,63 @@ __device__ __forceinline__ float cell_at(float step, uint32_t k) {
     return k ? __fmul_rn(step, __uint2float_rn(k)) : 0.0f;
 }
 
-template <bool GRID>
-__global__ __launch_bounds__(kSampleThreads) void k_cell_coarse(const float* __restrict__ cmf,
-                                                                uint32_t n, uint32_t G,
-                                                                uint32_t* __restrict__ coarse) {
-    pdl_entry();
-    const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= coarse_entries(G)) return;
-    const uint64_t k = static_cast<uint64_t>(j) * kCoarseStride;
-    coarse[j] = k < G ? bisect(cmf, 0, n - 1u,
-                               cell_at(cell_step<GRID>(cmf, n, G), static_cast<uint32_t>(k)))
-                      : n - 1u;
+//
+// The first pass is one thread per group that waits for each probe, so it reads the seven midpoints
+// that the next three levels may probe together (bisect_ahead: bisect's probes and result on any CMF).
+// n = 2^22, 4096 groups (the Cutpoint configuration's pass): a pass over every 1024th start and one
+// inside its brackets, a probe at a time, 185.9 us; both three levels at a time 182.1 (two: 182.2,
+// four: 184.1); one pass over the whole CMF 177.8.  ITS grid of 2^24 weights 535.6, 530, 523.4; of 2^27
+// (512 K groups) a build 920 with the pass between, 913 without: it is gone.
+__device__ __forceinline__ uint32_t bisect_ahead(const float* __restrict__ cmf, uint32_t x,
+                                                 uint32_t y, float u) {
+    constexpr int kLevels = 3, kNodes = (1 << kLevels) - 1;  // node k's children: 2k + 1 (down), 2k + 2 (up)
+    while (x < y) {
+        uint32_t lo[kNodes], hi[kNodes];
+        float v[kNodes];
+        lo[0] = x;
+        hi[0] = y;
+#pragma unroll
+        for (int k = 0; k < kNodes; ++k) {
+            const uint32_t mid = lo[k] + ((hi[k] - lo[k]) >> 1);
+            const bool live = lo[k] < hi[k];
+            v[k] = live ? __ldg(cmf + mid) : 0.f;
+            if (2 * k + 2 < kNodes) {  // (a dead node's children: dead)
+                lo[2 * k + 1] = lo[k];
+                hi[2 * k + 1] = mid;
+                lo[2 * k + 2] = live ? mid + 1u : lo[k];
+                hi[2 * k + 2] = hi[k];
+            }
+        }
+        int at = 0;  // the node's place in its level
+#pragma unroll
+        for (int level = 0; level < kLevels; ++level) {
+            if (x >= y) break;
+            float c = v[(1 << level) - 1];
+#pragma unroll
+            for (int q = 1; q < 1 << level; ++q) c = at == q ? v[(1 << level) - 1 + q] : c;
+            const uint32_t mid = x + ((y - x) >> 1);
+            const bool up = u > c;
+            if (up)
+                x = mid + 1u;
+            else
+                y = mid;
+            at = 2 * at + (up ? 1 : 0);
+        }
+    }
+    return x;
 }
-
-template <bool GRID>
-__device__ __forceinline__ uint32_t cell_start(const float* __restrict__ cmf, uint32_t n,
-                                               uint32_t G, const uint32_t* __restrict__ coarse,
-                                               uint32_t k) {
-    const uint32_t j = k / kCoarseStride;
-    const uint32_t lo = __ldg(coarse + j);
-    if (k % kCoarseStride == 0u) return lo;
-    return bisect(cmf, lo, __ldg(coarse + j + 1u), cell_at(cell_step<GRID>(cmf, n, G), k));
-}
-
 // group[g] = x_{32 g} (N - 1 past the last cell), g <= ceil(G / 32)
 template <bool GRID>
 __global__ __launch_bounds__(kSampleThreads) void k_cell_groups(const float* __restrict__ cmf,
                                                                 uint32_t n, uint32_t G,
-                                                                const uint32_t* __restrict__ coarse,
                                                                 uint32_t* __restrict__ group) {
     pdl_entry();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g >= group_entries(G)) return;
     const uint64_t k = static_cast<uint64_t>(g) * 32u;
-    group[g] = k < G ? cell_start<GRID>(cmf, n, G, coarse, static_cast<uint32_t>(k)) : n - 1u;
+    group[g] = k < G ? bisect_ahead(cmf, 0, n - 1u,
+                                    cell_at(cell_step<GRID>(cmf, n, G), static_cast<uint32_t>(k)))
+                     : n - 1u;
 }
 
 // The start of cell k = 32 g + lane (all lanes of the warp call it; k >= G returns N - 1), and
@@ -1342,18 +1364,12 @@ __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* 
     if (k < G) guide[k] = x;
 }
 
-// the first two passes: coarse starts, then group starts (scratch: coarse_entries(G) +
-// group_entries(G) words); returns the group array
+// the first pass (group: group_entries(G) words)
 template <bool GRID>
-static uint32_t* launch_cell_brackets(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                                      uint32_t* scratch) {
-    const uint32_t m = coarse_entries(G), ng = group_entries(G);
-    uint32_t* group = scratch + m;
-    launch_pdl(k_cell_coarse<GRID>, (m + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, cmf, n, G,
-                                                                                        scratch);
-    launch_pdl(k_cell_groups<GRID>, (ng + kSampleThreads - 1) / kSampleThreads, kSampleThreads, 0, st, 
-        cmf, n, G, scratch, group);
-    return group;
+static void launch_cell_groups(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
+                               uint32_t* group) {
+    launch_pdl(k_cell_groups<GRID>, (group_entries(G) + kSampleThreads - 1) / kSampleThreads,
+               kSampleThreads, 0, st, cmf, n, G, group);
 }
 
 static uint32_t warp_blocks(uint32_t G) {
@@ -1362,15 +1378,15 @@ static uint32_t warp_blocks(uint32_t G) {
 }
 
 cudaError_t launch_its_cells(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsCell* cells) {
-    uint32_t* group = launch_cell_brackets<false>(st, cmf, n, G, coarse);
+                             uint32_t* group, ItsCell* cells) {
+    launch_cell_groups<false>(st, cmf, n, G, group);
     launch_pdl(k_its_cells, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
     return cudaGetLastError();
 }
 
 cudaError_t launch_its_grids(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                             uint32_t* coarse, ItsGrid* grids) {
-    uint32_t* group = launch_cell_brackets<true>(st, cmf, n, G, coarse);
+                             uint32_t* group, ItsGrid* grids) {
+    launch_cell_groups<true>(st, cmf, n, G, group);
     launch_pdl(k_its_grids, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, grids);
     return cudaGetLastError();
 }
@@ -1581,8 +1597,8 @@ cudaError_t launch_cutpoint_guide(cudaStream_t st, const float* cmf, uint32_t n,
 }
 
 cudaError_t launch_guide_monotone(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
-                                  uint32_t* coarse, uint32_t* guide) {
-    uint32_t* group = launch_cell_brackets<false>(st, cmf, n, G, coarse);
+                                  uint32_t* group, uint32_t* guide) {
+    launch_cell_groups<false>(st, cmf, n, G, group);
     launch_pdl(k_guide_monotone, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, guide);
     return cudaGetLastError();
 }
