@@ -796,27 +796,40 @@ __device__ __forceinline__ uint32_t bisect_ahead(const float* __restrict__ cmf, 
 }
 // group[g] = x_{32 g} (N - 1 past the last cell), g <= ceil(G / 32)
 template <bool GRID>
+__device__ __forceinline__ uint32_t group_start(const float* __restrict__ cmf, uint32_t n, uint32_t G,
+                                                uint32_t g) {
+    const uint64_t k = static_cast<uint64_t>(g) * 32u;
+    return k < G ? bisect_ahead(cmf, 0, n - 1u,
+                                cell_at(cell_step<GRID>(cmf, n, G), static_cast<uint32_t>(k)))
+                 : n - 1u;
+}
+template <bool GRID>
 __global__ __launch_bounds__(kSampleThreads) void k_cell_groups(const float* __restrict__ cmf,
                                                                 uint32_t n, uint32_t G,
                                                                 uint32_t* __restrict__ group) {
     pdl_entry();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= group_entries(G)) return;
-    const uint64_t k = static_cast<uint64_t>(g) * 32u;
-    group[g] = k < G ? bisect_ahead(cmf, 0, n - 1u,
-                                    cell_at(cell_step<GRID>(cmf, n, G), static_cast<uint32_t>(k)))
-                     : n - 1u;
+    if (g < group_entries(G)) group[g] = group_start<GRID>(cmf, n, G, g);
 }
 
 // The start of cell k = 32 g + lane (all lanes of the warp call it; k >= G returns N - 1), and
-// the end of the group's bracket in hi.
-template <bool GRID>
+// the end of the group's bracket in hi.  OWN: without the first pass, the bracket's ends by the first
+// two lanes' bisections.
+template <bool GRID, bool OWN>
 __device__ __forceinline__ uint32_t cell_start_warp(const float* __restrict__ cmf, uint32_t n,
                                                     uint32_t G, const uint32_t* __restrict__ group,
                                                     uint32_t g, uint32_t& hi) {
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t lo = __ldg(group + g);
-    hi = __ldg(group + g + 1u);
+    uint32_t lo;
+    if constexpr (OWN) {
+        uint32_t end = 0;
+        if (lane < 2u) end = group_start<GRID>(cmf, n, G, g + lane);
+        lo = __shfl_sync(0xffffffffu, end, 0);
+        hi = __shfl_sync(0xffffffffu, end, 1);
+    } else {
+        lo = __ldg(group + g);
+        hi = __ldg(group + g + 1u);
+    }
     const uint32_t k = g * 32u + lane;
     const float t = k < G ? cell_at(cell_step<GRID>(cmf, n, G), k) : __int_as_float(0x7f800000);
     uint32_t x;
@@ -864,6 +877,7 @@ __device__ __forceinline__ uint32_t cell_part(uint32_t x, uint32_t y) {
 
 // the FP32 CMF need not be monotone: a cell whose start x > 0 does not have cmf[x - 1] < c_k is
 // marked for the bisection as it is written
+template <bool OWN>
 __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __restrict__ cmf,
                                                               uint32_t n, uint32_t G,
                                                               const uint32_t* __restrict__ group,
@@ -872,7 +886,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __res
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
-    const uint32_t x = cell_start_warp<false>(cmf, n, G, group, g, hi);
+    const uint32_t x = cell_start_warp<false, OWN>(cmf, n, G, group, g, hi);
     const uint32_t k = g * 32u + (threadIdx.x & 31u);
     // the end of a cell is the next cell's start: the next lane's, or the next group's
     uint32_t y = __shfl_down_sync(0xffffffffu, x, 1);
@@ -904,6 +918,7 @@ __device__ __forceinline__ uint32_t grid_f(float v, float scale) {
 // One cell per lane, a warp per 32 (cell_start_warp finds their starts): the steps of its parts'
 // last items.  0.051 ms at n = 2^24 (2^21 cells, 64 MB written, the CMF read once from HBM: 2.6
 // TB/s), issue-bound: 27 loads and conversions a cell.
+template <bool OWN>
 __global__ __launch_bounds__(kSampleThreads) void k_its_grids(const float* __restrict__ cmf,
                                                               uint32_t n, uint32_t G,
                                                               const uint32_t* __restrict__ group,
@@ -912,7 +927,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_grids(const float* __res
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
-    const uint32_t x = cell_start_warp<true>(cmf, n, G, group, g, hi);
+    const uint32_t x = cell_start_warp<true, OWN>(cmf, n, G, group, g, hi);
     const uint32_t k = g * 32u + (threadIdx.x & 31u);
     uint32_t y = __shfl_down_sync(0xffffffffu, x, 1);
     if ((threadIdx.x & 31u) == 31u) y = hi;
@@ -1351,6 +1366,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_cells(
 // Guiding table of an exactly non-decreasing CMF: the same entries as k_cutpoint_guide
 // (guide[k] = lower bound of fl(fl(total / G) * k), clamped to N - 1), where every lower-bound
 // search gives the same index, so the bracketed searches of cell_start apply.
+template <bool OWN>
 __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* __restrict__ cmf,
                                                                    uint32_t n, uint32_t G,
                                                                    const uint32_t* __restrict__ group,
@@ -1359,17 +1375,25 @@ __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* 
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
-    const uint32_t x = cell_start_warp<false>(cmf, n, G, group, g, hi);
+    const uint32_t x = cell_start_warp<false, OWN>(cmf, n, G, group, g, hi);
     const uint32_t k = g * 32u + (threadIdx.x & 31u);
     if (k < G) guide[k] = x;
 }
 
-// the first pass (group: group_entries(G) words)
+// Up to this many cells the second pass's warps find their brackets themselves: a launch less, and
+// few enough warps that all wait at once.  Builds, with the first pass / without: ITS n = 65536 (8192
+// cells) 26.5 / 24.2 us, n = 5000 22.6 / 20.9, n = 4 x 10^6 (500 K) 53.3 / 57.2; Cutpoint, entry 32, n =
+// 10^5 (3125) 25.2 / 24.3, n = 2^22 (131072) 44.3 / 47.4.
+constexpr uint32_t kOwnMaxCells = 32768;
+
+// the first pass (group: group_entries(G) words); true: left to the second
 template <bool GRID>
-static void launch_cell_groups(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
+static bool launch_cell_groups(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                uint32_t* group) {
+    if (G <= kOwnMaxCells) return true;
     launch_pdl(k_cell_groups<GRID>, (group_entries(G) + kSampleThreads - 1) / kSampleThreads,
                kSampleThreads, 0, st, cmf, n, G, group);
+    return false;
 }
 
 static uint32_t warp_blocks(uint32_t G) {
@@ -1379,15 +1403,15 @@ static uint32_t warp_blocks(uint32_t G) {
 
 cudaError_t launch_its_cells(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                              uint32_t* group, ItsCell* cells) {
-    launch_cell_groups<false>(st, cmf, n, G, group);
-    launch_pdl(k_its_cells, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
+    const bool own = launch_cell_groups<false>(st, cmf, n, G, group);
+    launch_pdl(own ? k_its_cells<true> : k_its_cells<false>, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, cells);
     return cudaGetLastError();
 }
 
 cudaError_t launch_its_grids(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                              uint32_t* group, ItsGrid* grids) {
-    launch_cell_groups<true>(st, cmf, n, G, group);
-    launch_pdl(k_its_grids, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, grids);
+    const bool own = launch_cell_groups<true>(st, cmf, n, G, group);
+    launch_pdl(own ? k_its_grids<true> : k_its_grids<false>, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, grids);
     return cudaGetLastError();
 }
 
@@ -1598,8 +1622,8 @@ cudaError_t launch_cutpoint_guide(cudaStream_t st, const float* cmf, uint32_t n,
 
 cudaError_t launch_guide_monotone(cudaStream_t st, const float* cmf, uint32_t n, uint32_t G,
                                   uint32_t* group, uint32_t* guide) {
-    launch_cell_groups<false>(st, cmf, n, G, group);
-    launch_pdl(k_guide_monotone, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, guide);
+    const bool own = launch_cell_groups<false>(st, cmf, n, G, group);
+    launch_pdl(own ? k_guide_monotone<true> : k_guide_monotone<false>, warp_blocks(G), kSampleThreads, 0, st, cmf, n, G, group, guide);
     return cudaGetLastError();
 }
 
