@@ -295,6 +295,10 @@ struct PartX {
     u128 h, l;
     uint32_t c;
 };
+struct PartOne {  // one class of it (c: heavy only)
+    u128 x;
+    uint32_t c;
+};
 
 __device__ __forceinline__ PartCarry part_sum_f(PartCarry v) {
 #pragma unroll
@@ -315,30 +319,36 @@ __device__ __forceinline__ PartX part_sum_x(PartX v) {
     return v;
 }
 
-__device__ PartX part_lookback_x(const PartState* st, uint32_t tile, uint32_t first,
-                                 uint32_t* status, uint32_t spin_limit) {
-    const PartX zero{0, 0, 0u};
+// The exact lookback of one class: warp 0 walks back over the heavy sums and counts, warp 1 over the
+// light sums, at once.
+__device__ PartOne part_lookback_x(const PartState* st, bool heavy, uint32_t tile, uint32_t first,
+                                   uint32_t* status, uint32_t spin_limit) {
+    const PartOne zero{0, 0u};
+    const uint32_t at = heavy ? 0u : 2u;
     return lookback_walk(
         tile, first, status, spin_limit, zero,
-        [st](uint32_t pos, PartX& v) -> int {
+        [st, at, heavy](uint32_t pos, PartOne& v) -> int {
             // inclusive words first; the aggregate only where those are not yet published
             const unsigned long long* q = st[pos].q;
-            unsigned long long h0, h1, l0, l1, c, pad;
-            ld_relaxed_v2(q + 8, h0, h1);
-            ld_relaxed_v2(q + 10, l0, l1);
-            ld_relaxed_v2(q + 6, c, pad);
+            unsigned long long x0, x1, c = pack_cnt(0u), pad;
+            ld_relaxed_v2(q + 8 + at, x0, x1);
+            if (heavy) ld_relaxed_v2(q + 6, c, pad);
             int s = 2;
-            if (!(fx_ready(h0, h1) && fx_ready(l0, l1) && cnt_ready(c))) {
-                ld_relaxed_v2(q + 0, h0, h1);
-                ld_relaxed_v2(q + 2, l0, l1);
-                ld_relaxed_v2(q + 4, c, pad);
-                s = fx_ready(h0, h1) && fx_ready(l0, l1) && cnt_ready(c) ? 1 : 0;
+            if (!(fx_ready(x0, x1) && cnt_ready(c))) {
+                ld_relaxed_v2(q + at, x0, x1);
+                if (heavy) ld_relaxed_v2(q + 4, c, pad);
+                s = fx_ready(x0, x1) && cnt_ready(c) ? 1 : 0;
             }
-            if (s) v = {fx_unpack(h0, h1), fx_unpack(l0, l1), static_cast<uint32_t>(c)};
+            if (s) v = {fx_unpack(x0, x1), static_cast<uint32_t>(c)};
             return s;
         },
-        [](PartX v) { return part_sum_x(v); },
-        [](PartX a, PartX b) { return PartX{a.h + b.h, a.l + b.l, a.c + b.c}; });
+        [heavy](PartOne v) {
+#pragma unroll
+            for (int m = 1; m < 32; m <<= 1) v.x += shfl_xor_u128(v.x, m);
+            if (heavy) v.c = __reduce_add_sync(0xffffffffu, v.c);
+            return v;
+        },
+        [](PartOne a, PartOne b) { return PartOne{a.x + b.x, a.c + b.c}; });
 }
 
 __device__ PartCarry part_lookback_f(const PartState* st, uint32_t tile, uint32_t first,
@@ -366,11 +376,9 @@ __device__ PartCarry part_lookback_f(const PartState* st, uint32_t tile, uint32_
         });
 }
 
-__device__ __forceinline__ void part_publish_x(PartState* s, const PartX& a, bool incl) {
-    unsigned long long* q = s->q + (incl ? 8 : 0);
-    st_relaxed_v2(q + 0, fx_word_lo(a.h), fx_word_hi(a.h));
-    st_relaxed_v2(q + 2, fx_word_lo(a.l), fx_word_hi(a.l));
-    st_relaxed(s->q + (incl ? 6 : 4), pack_cnt(a.c));
+__device__ __forceinline__ void part_publish_x(PartState* s, bool heavy, const PartOne& a, bool incl) {
+    st_relaxed_v2(s->q + (incl ? 8 : 0) + (heavy ? 0 : 2), fx_word_lo(a.x), fx_word_hi(a.x));
+    if (heavy) st_relaxed(s->q + (incl ? 6 : 4), pack_cnt(a.c));
 }
 __device__ __forceinline__ void part_publish_f(PartState* s, const PartCarry& a, bool incl) {
     st_relaxed_v2(s->q + (incl ? 8 : 0), pack_ff(ff{a.h, 0.f}), pack_ff(ff{a.l, 0.f}));
@@ -552,9 +560,58 @@ __device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchVie
     }
     __syncthreads();
 
-    // ---- phase B (warp 0): warp-exclusive offsets, tile aggregate, lookback
+    // ---- phase B (warp 0, or warps 0 and 1): warp-exclusive offsets, tile aggregate, lookback
     uint32_t left = 0xffffffffu;
-    if (warp == 0) {
+    constexpr bool TWO = COMP && CARRY == Carry::kLookback;
+    if constexpr (TWO) {
+        // The heavy class by warp 0, the light one by warp 1: while they walk back the CTA's other
+        // warps wait, and a window of the walk takes as long as its loads and its 126-bit sums (2^26
+        // weights, both classes by one warp: float-float 430 -> 413 us, compensated 333 -> 320; 2^24 124
+        // -> 121 and 96 -> 92).
+        if (warp < 2) {
+            const bool heavy = warp == 0;
+            ff agg{0.f, 0.f}, exw{0.f, 0.f};
+            float ew = 0.f;
+            if constexpr (FFOUT) {
+                const ff it = ff_warp_incl(
+                    lane < kTileWarps ? (heavy ? s_fh : s_fl)[lane] : ff{0.f, 0.f}, lane);
+                exw = ff_shfl_up_excl(it, lane);
+                agg = ff_shfl(it, kTileWarps - 1);
+            } else {
+                const float it =
+                    warp_incl_f(lane < kTileWarps ? (heavy ? s_wh : s_wl)[lane] : 0.f, lane);
+                ew = __shfl_up_sync(0xffffffffu, it, 1);
+                agg = {__shfl_sync(0xffffffffu, it, kTileWarps - 1), 0.f};
+            }
+            uint32_t agg_c = 0, ec = 0;
+            if (heavy) {
+                const uint32_t ic = warp_incl_u(lane < kTileWarps ? s_wc[lane] : 0u, lane);
+                ec = __shfl_up_sync(0xffffffffu, ic, 1);
+                agg_c = __shfl_sync(0xffffffffu, ic, kTileWarps - 1);
+            }
+            __syncwarp();
+            if (lane < kTileWarps) {
+                if (heavy) s_wc[lane] = lane ? ec : 0u;
+                if constexpr (FFOUT)
+                    (heavy ? s_fh : s_fl)[lane] = exw;
+                else
+                    (heavy ? s_wh : s_wl)[lane] = lane ? ew : 0.f;
+            }
+            const int grid = fx_grid(ctrl->total);
+            const PartOne mine{fx_from_ff(agg, grid), agg_c};
+            PartOne ex{0, 0u};
+            if (lane == 0) part_publish_x(cur + tile, heavy, mine, false);
+            if (tile != first) ex = part_lookback_x(cur, heavy, tile, first, a.status, a.spin_limit);
+            if (lane == 0) {
+                part_publish_x(cur + tile, heavy, PartOne{ex.x + mine.x, ex.c + agg_c}, true);
+                (heavy ? s_exh : s_exl) = fx_to_ff(ex.x, grid);
+                if (heavy) {
+                    s_exc = ex.c;
+                    s_aggc = agg_c;
+                }
+            }
+        }
+    } else if (warp == 0) {
         const uint32_t ic = warp_incl_u(lane < kTileWarps ? s_wc[lane] : 0u, lane);
         const uint32_t ec = __shfl_up_sync(0xffffffffu, ic, 1);
         const uint32_t agg_c = __shfl_sync(0xffffffffu, ic, kTileWarps - 1);
@@ -595,26 +652,6 @@ __device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchVie
             exh = {__ldg(a.bw_h + tile), 0.f};
             exl = {__ldg(a.bw_l + tile), 0.f};
             exc = __ldg(a.bw_c + tile);
-        } else if constexpr (COMP) {
-            const int grid = fx_grid(ctrl->total);
-            const PartX agg{fx_from_ff(agg_h, grid), fx_from_ff(agg_l, grid), agg_c};
-            PartX ex{0, 0, 0u};
-            if (tile == first) {
-                if (lane == 0) {
-                    part_publish_x(cur + tile, agg, false);
-                    part_publish_x(cur + tile, agg, true);
-                }
-            } else {
-                if (lane == 0) part_publish_x(cur + tile, agg, false);
-                ex = part_lookback_x(cur, tile, first, a.status, a.spin_limit);
-                if (lane == 0)
-                    part_publish_x(cur + tile, PartX{ex.h + agg.h, ex.l + agg.l, ex.c + agg.c}, true);
-            }
-            if (lane == 0) {
-                exh = fx_to_ff(ex.h, grid);
-                exl = fx_to_ff(ex.l, grid);
-            }
-            exc = ex.c;
         } else {
             const PartCarry agg{agg_h.hi, agg_l.hi, agg_c};
             PartCarry ex{0.f, 0.f, 0u};
@@ -680,6 +717,9 @@ __device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchVie
         }
     }
     __syncthreads();
+
+    if constexpr (TWO)
+        if (threadIdx.x == 0) left = lookback_leave(a.lb);  // (both warps' lookbacks have ended)
 
     // ---- phase C: running sums over the thread's items, staged by output slot, written out
     const uint32_t tbase = lt * kTileItems;
