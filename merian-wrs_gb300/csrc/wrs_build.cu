@@ -343,8 +343,7 @@ __device__ PartOne part_lookback_x(const PartState* st, bool heavy, uint32_t til
             return s;
         },
         [heavy](PartOne v) {
-#pragma unroll
-            for (int m = 1; m < 32; m <<= 1) v.x += shfl_xor_u128(v.x, m);
+            v.x = warp_sum_u126(v.x);
             if (heavy) v.c = __reduce_add_sync(0xffffffffu, v.c);
             return v;
         },
@@ -1068,11 +1067,7 @@ __device__ u128 scan_lookback_x(const ScanState* st, uint32_t tile, uint32_t* st
             if (s) v = fx_unpack(lo, hi);
             return s;
         },
-        [](u128 v) {
-#pragma unroll
-            for (int m = 1; m < 32; m <<= 1) v += shfl_xor_u128(v, m);
-            return v;
-        },
+        [](u128 v) { return warp_sum_u126(v); },
         [](u128 a, u128 b) { return a + b; });
 }
 

@@ -263,6 +263,20 @@ __device__ __forceinline__ u128 fx_unpack(unsigned long long lo, unsigned long l
     return (static_cast<u128>(hi & kLimbMask) << 63) | (lo & kLimbMask);
 }
 
+// The warp's sum of values below 2^126 (mod 2^128; every lane gets it): pieces of 26 bits, whose sums
+// over 32 lanes fit in 32 bits, by the warp's integer reduction.  On the lookbacks' critical path (five
+// rounds of four shuffles and a carry chain before: exact scan and ITS pass of 2^24 weights 525.1 -> 521.6
+// us, float-float partition of 2^26 414 -> 411).
+__device__ __forceinline__ u128 warp_sum_u126(u128 v) {
+    u128 sum = 0;
+#pragma unroll
+    for (int p = 0; p < 5; ++p) {
+        const uint32_t piece = static_cast<uint32_t>(v >> (26 * p)) & 0x3ffffffu;
+        sum += static_cast<u128>(__reduce_add_sync(0xffffffffu, piece)) << (26 * p);
+    }
+    return sum;
+}
+
 // ---------------------------------------------------------------------------
 // lookback words.  An ff word is {hi bits, lo bits | 1}: the LSB of lo's
 // mantissa is the ready bit (the value loses at most one ulp of lo).  A count
