@@ -1054,7 +1054,9 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_grids(
                     y = mid;
             }
         } else if (same) {
-            while (x < last && t[v] > __ldg(cmf + x)) ++x;
+            // (the cell's items end before y on the CMF it was built from; on any other the walk ends)
+            const uint32_t y = min(x0 + static_cast<uint32_t>(kGridSlots), last);
+            while (x < y && t[v] > __ldg(cmf + x)) ++x;
         }
         res[v] = x;
     }
