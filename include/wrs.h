@@ -185,7 +185,11 @@ void wrs_destroy(wrs_handle* h);
  * per weight up to 2^26 in all): wrs_build writes them after the table and wrs_sample reads them for
  * the n built last, so that most samples skip the table read (same samples; wrs_split_pack and
  * wrs_pack into the buffers retire them until the next build, and the primitive wrs_alias_sample
- * reads the table alone). */
+ * reads the table alone).  ITS and Cutpoint: what a build stores beside the CMF is retired in the
+ * same way by wrs_prefix_sum and wrs_prefix_sum_blockwise over any of the CMF in these buffers; the
+ * samples that follow bisect.  All of this is noted on the host, in the order of the calls: after a
+ * table or CMF has changed in another way (the caller's own copy, a primitive given other buffers, a
+ * graph replayed out of that order) build again, or sample with the primitives. */
 size_t wrs_buffers_bytes(const wrs_handle* h, uint32_t max_n);
 wrs_status wrs_buffers_create(const wrs_handle* h, uint32_t max_n, wrs_buffers** out);
 void wrs_buffers_destroy(wrs_buffers* b);

@@ -321,6 +321,21 @@ static wrs_status check_n(const wrs_buffers* b, uint32_t n) {
     return WRS_OK;
 }
 
+// What a build stored beside the CMF for the sampler's search (cells or grid, probe tree, the CMF's
+// monotonicity) holds for that CMF alone: a primitive that writes out[0, n) over any of it retires
+// them, and the next samples bisect.
+static void retire_search(wrs_buffers* b) {
+    b->monotone_n = 0;
+    b->cells_n = 0;
+    b->tree_n = 0;
+}
+static void retire_overwritten(wrs_buffers* b, const float* out, uint32_t n) {
+    const uintptr_t o = reinterpret_cast<uintptr_t>(out), c = reinterpret_cast<uintptr_t>(b->cmf);
+    if (b->cmf && o < c + sizeof(float) * static_cast<size_t>(b->max_n) &&
+        c < o + sizeof(float) * static_cast<size_t>(n))
+        retire_search(b);
+}
+
 wrs_status wrs_total_mass(const wrs_handle* h, void* stream, const float* weights, uint32_t n,
                           wrs_buffers* b) {
     if (!h || !weights) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
@@ -335,7 +350,7 @@ wrs_status wrs_prefix_sum(const wrs_handle* h, void* stream, const float* in, ui
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
-    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
+    retire_overwritten(b, out, n);
     WRS_CUDA(launch_scan(as_stream(stream), h->cfg.scan_precision != WRS_SCAN_FP32, in, n,
                          out, b->ctrl, b->scan_states, b->cap_tiles, b->partials),
              "prefix sum");
@@ -413,7 +428,7 @@ wrs_status wrs_prefix_sum_blockwise(const wrs_handle* h, void* stream, const flo
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
-    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
+    retire_overwritten(b, out, n);
     WRS_CUDA(launch_prefix_sum_blockwise(as_stream(stream), in, n, out,
                                          reinterpret_cast<float*>(b->tile_scratch)),
              "block-wise prefix sum");
@@ -543,7 +558,7 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
     const cudaStream_t st = as_stream(stream);
     const bool comp = compensated(h);
     if (h->cfg.method != WRS_METHOD_ALIAS_TABLE) {
-        b->monotone_n = 0;
+        retire_search(b);
         WRS_CUDA(launch_scan(st, comp, weights, n, b->cmf, b->ctrl, b->scan_states, b->cap_tiles,
                              b->partials),
                  "ITS build");
@@ -556,7 +571,6 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
                           : launch_cutpoint_guide(st, b->cmf, n, G, b->guide),
                      "guiding table");
         else if (its_guided(h)) {
-            b->cells_n = 0;
             b->cells_grid = comp;
             if (comp) {
                 WRS_CUDA(launch_its_grids(st, b->cmf, n, its_grids(n, h->cfg.guiding_entry_size),
@@ -572,7 +586,6 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
             }
             b->cells_n = n;
         }
-        b->tree_n = 0;
         if (b->tree && its_tree_levels(h->cfg, n)) {
             WRS_CUDA(launch_its_tree(st, b->cmf, n, its_tree_stored_levels(n), b->tree),
                      "ITS probe tree");
@@ -724,7 +737,7 @@ wrs_status wrs_test_prefix_sum_stalled(const wrs_handle* h, void* stream, const 
     if (!h || !in || !out) return fail(WRS_ERR_INVALID_ARG, "NULL argument");
     wrs_status s = check_n(b, n);
     if (s != WRS_OK) return s;
-    if (out == b->cmf) b->monotone_n = 0;  // no longer known to be the build's
+    retire_overwritten(b, out, n);
     if (spin_limit == 0 || spin_limit > kSpinLimit)
         return fail(WRS_ERR_INVALID_ARG, "spin_limit out of range");
     const cudaStream_t st = as_stream(stream);
