@@ -982,7 +982,15 @@ constexpr int kGridPerThread = 2;
 // 0.91 -> 0.34 (195 G/s; issue 72 % active, 145 instructions per 32 samples), against the FP32 cells'
 // six values and index range (8 bytes per weight, 332 instructions); n = 2^26, 2^27 samples: uniform
 // 2.46 -> 1.10, log-normal 2.78 -> 1.80 ms (the grid exceeds L2: random HBM reads again).
-template <uint32_t RNG>
+//
+// CACHED: a grid that fits the L1s is read through them.  A small one read around them comes from a
+// few L2 sectors that every SM asks for: n = 1000 uniform, 2^24 samples 541 us around, 109 through
+// (199 by the FP32 cells); n = 10^4 132 and 108, n = 2 * 10^4 (78 KB) 182 and 111.  At 156 KB both take
+// 103; a larger one only pushes the CMF values out (64 MB, the shaders' stream, 2^26 samples: 586 and
+// 604; n = 10^6 with entry 64, 244 KB, 794 and 829).
+constexpr uint32_t kGridCachedMax = 4096;  // cells: 128 KB
+
+template <uint32_t RNG, bool CACHED>
 __global__ __launch_bounds__(kSampleThreads) void k_its_sample_grids(
     const float* __restrict__ cmf, uint32_t n, const ItsGrid* __restrict__ grids, uint32_t G,
     uint64_t S, uint64_t seed, uint64_t offset, uint32_t* __restrict__ out) {
@@ -1017,7 +1025,11 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_grids(
 #pragma unroll
     for (int v = 0; v < kGridPerThread; ++v) {
         F[v] = grid_f(t[v], scale);
-        ld_block(reinterpret_cast<const uint32_t*>(grids + min(F[v] >> 7, G - 1u)), lo[v], hi[v]);
+        const uint32_t* cell = reinterpret_cast<const uint32_t*>(grids + min(F[v] >> 7, G - 1u));
+        if constexpr (CACHED)
+            ld_u32x8(cell, lo[v], hi[v]);
+        else
+            ld_block(cell, lo[v], hi[v]);
     }
 #pragma unroll
     for (int v = 0; v < kGridPerThread; ++v) {
@@ -1424,12 +1436,15 @@ cudaError_t launch_its_sample_grids(cudaStream_t st, uint32_t rng, const float* 
     const uint64_t grid = (S + per - 1) / per;
     if (grid == 0) return cudaSuccess;
     if (grid > 0x7fffffffull) return cudaErrorInvalidValue;
+    const bool cached = G <= kGridCachedMax;
+    auto go = [&](auto kernel) {
+        launch_pdl(kernel, static_cast<unsigned>(grid), kSampleThreads, 0, st, cmf, n, grids, G, S, seed,
+                   offset, out);
+    };
     if (rng == RNG_REF)
-        launch_pdl(k_its_sample_grids<RNG_REF>, static_cast<unsigned>(grid), kSampleThreads, 0, st,
-                   cmf, n, grids, G, S, seed, offset, out);
+        cached ? go(k_its_sample_grids<RNG_REF, true>) : go(k_its_sample_grids<RNG_REF, false>);
     else
-        launch_pdl(k_its_sample_grids<RNG_PHILOX>, static_cast<unsigned>(grid), kSampleThreads, 0,
-                   st, cmf, n, grids, G, S, seed, offset, out);
+        cached ? go(k_its_sample_grids<RNG_PHILOX, true>) : go(k_its_sample_grids<RNG_PHILOX, false>);
     return cudaGetLastError();
 }
 

@@ -51,3 +51,23 @@ def test_grid_equals_the_bisection(pkg, cuda, n, entry, gen, scale, rng):
         cuda.cuda.synchronize()
         assert cuda.equal(out[0], out[1])
         assert int(got.min()) >= 0 and int(got.max()) < n
+
+
+@pytest.mark.parametrize("rng", [0, 1])
+@pytest.mark.parametrize("n", [4 * 8192 - 7, 4 * 8192, 4 * 8192 + 1])
+def test_grid_around_the_cached_size(pkg, cuda, n, rng):
+    """Grids of up to 4096 cells are read through the L1s, larger ones around them."""
+    W = pkg.wrs
+    cfg = W.ITSConfig(rng=rng, scan_precision=W.SCAN_COMPENSATED)
+    wrs = W.WRS(cfg)
+    b = W.WRSBuffers.allocate(n, 1, cfg, handle=wrs.handle)
+    s = 200_001
+    out = cuda.full((2, s), -1, dtype=cuda.int32, device="cuda")
+    for seed in (1, 2):  # the second build's grid, not the first one's lines
+        b.weights.copy_(h2d(weights_lognormal(n, seed)))
+        wrs.build(None, b, n)
+        W.check(W.lib().wrs_sample_at(wrs.handle.ptr, None, b.internals.ptr, n, s, 9, 0,
+                                      out[0].data_ptr()))
+        wrs.its_sample(None, b.internals.views()["cmf"], n, s, 9, 0, out[1].data_ptr())
+        cuda.cuda.synchronize()
+        assert cuda.equal(out[0], out[1])
