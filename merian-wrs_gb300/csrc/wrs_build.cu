@@ -123,7 +123,7 @@ __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __rest
                                                              double* __restrict__ partials,
                                                              BuildCtrl* __restrict__ ctrl_in,
                                                              BatchView bv) {
-    pdl_entry();
+    pdl_wait();
     __shared__ double s_red[kTileWarps];
     __shared__ ff s_part[kTileWarps];
     __shared__ bool s_last;
@@ -844,7 +844,7 @@ __device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchVie
 template <bool COMP, bool FFOUT, bool BATCH, bool BW = false>
 __global__ __launch_bounds__(kTileThreads, kPartMinBlocks) void k_prefix_partition(PartArgs a,
                                                                                    BatchView bv) {
-    pdl_entry();
+    pdl_wait();
     __shared__ __align__(16) unsigned char s_raw[kPartBytes];
     partition_tile<COMP, FFOUT, BATCH, BW ? Carry::kGiven : Carry::kLookback>(a, bv, s_raw,
                                                                               ClusterPart{});
@@ -924,7 +924,7 @@ __global__ __launch_bounds__(kTileThreads) void k_scan_bulk(const float* __restr
                                                             ScanState* __restrict__ states,
                                                             uint32_t cap_tiles,
                                                             uint32_t spin_limit) {
-    pdl_entry();
+    pdl_wait();
     constexpr uint32_t kItems = kTileThreads * 4u * V;  // per tile
     constexpr uint32_t kWarpSpan = 128u * V;             // per warp
     extern __shared__ __align__(128) float s_tile[];     // kItems floats
@@ -1100,7 +1100,7 @@ __global__ __launch_bounds__(kTileThreads, 8) void k_scan_exact(const float* __r
                                                              ScanState* __restrict__ states,
                                                              uint32_t cap_tiles,
                                                              uint32_t spin_limit) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float4 s_x[kTileItems / 4];  // the tile (park_slot), later its outputs
     __shared__ u128 s_e[kTileThreads];       // exact thread-exclusive sums within the warp
     __shared__ u128 s_wt[kTileWarps];        // exact warp totals -> warp-exclusive sums
@@ -1866,7 +1866,7 @@ constexpr uint32_t kDescentThreads = 128;
 // (BATCH: one thread per split-pack CTA of the whole batch, each of its distribution)
 template <bool FF, bool BATCH>
 __global__ __launch_bounds__(kDescentThreads) void k_split_descent(SplitArgs a, BatchView bv) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;  // the split-pack CTA
     uint32_t blk = g, n = a.n;
     const BuildCtrl* ctrl = a.ctrl;
@@ -2095,7 +2095,7 @@ __device__ __forceinline__ void pack_cta(const P& c, uint2* table, uint32_t* sta
 // ownership window.
 template <bool R64, bool FF, bool BATCH, bool RECORDS = false>
 __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, BatchView bv) {
-    pdl_entry();
+    pdl_wait();
     __shared__ uint32_t s_i[kSplitSlots], s_j[kSplitSlots];
     const float* w = a.w;
     uint32_t n = a.n;
@@ -2239,7 +2239,7 @@ constexpr uint32_t kSmallStage = kPartBytes / 8u - 4u;  // staged words; as many
 
 template <bool R64, bool COMP, bool FFOUT>
 __global__ __launch_bounds__(kTileThreads, 1) void k_build_small(PartArgs a, SplitArgs sa) {
-    pdl_entry();
+    pdl_wait();
     cluster_arrive();
     __shared__ __align__(16) unsigned char s_raw[kPartBytes];
     __shared__ ff s_part[kTileWarps];
@@ -2458,7 +2458,7 @@ template <bool APPLY>
 __global__ __launch_bounds__(kTileThreads) void k_bw_scan(const float* __restrict__ in, uint32_t n,
                                                           float* __restrict__ out,
                                                           float* __restrict__ tile_val) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float s_w[kTileWarps];
     const uint32_t tile = blockIdx.x;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2519,7 +2519,7 @@ __global__ __launch_bounds__(kTileThreads) void k_bw_part_reduce(const float* __
                                                                  uint32_t* __restrict__ tc,
                                                                  float* __restrict__ th,
                                                                  float* __restrict__ tl) {
-    pdl_entry();
+    pdl_wait();
     __shared__ uint32_t s_c[kTileWarps];
     __shared__ float s_h[kTileWarps], s_l[kTileWarps];
     const uint32_t tile = blockIdx.x;
@@ -2570,7 +2570,7 @@ constexpr int kBwThreads = 1024;
 __global__ __launch_bounds__(kBwThreads) void k_bw_tiles(uint32_t T, uint32_t* __restrict__ c,
                                                          float* __restrict__ h,
                                                          float* __restrict__ l) {
-    pdl_entry();
+    pdl_wait();
     __shared__ uint32_t s_c[32];
     __shared__ float s_h[32], s_l[32];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -2664,7 +2664,7 @@ cudaError_t launch_prefix_partition_blockwise(cudaStream_t st, const float* w, u
 // light: every record is the final one (the shader's bisection would underflow).
 template <bool R64, bool FF>
 __global__ __launch_bounds__(256) void k_split_records(SplitArgs a) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t n = a.n;
     const uint32_t K = records_for(n, a.split_size);
     const uint32_t t = blockIdx.x * blockDim.x + threadIdx.x;  // record t: split k = t + 1
@@ -2762,7 +2762,7 @@ __device__ __forceinline__ bool covered_later_warp(uint32_t li, uint32_t lj, uin
 }
 
 __global__ __launch_bounds__(256) void k_pack_records_warp(SplitArgs a) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t k = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // subproblem
     const uint32_t n = a.n;

@@ -25,21 +25,17 @@ constexpr uint32_t kSpinLimit = 1u << 21;  // lookback polls before giving up (>
 constexpr uint32_t kCopyDrainLimit = 1u << 25;
 
 // Programmatic dependent launch.  A kernel launched with programmatic stream serialization
-// (launch_pdl) may be scheduled while the kernel before it in the stream still runs:
-// its CTAs wait here until that kernel has completed and its memory is visible, so the launch and the
-// CTAs' start overlap the predecessor's tail instead of following it.  A kernel of a build whose grid
-// is about one wave then lets its own dependent be scheduled at once; a larger one's is as its last
-// CTAs end, since CTAs that wait from early on take room from its own (a 2^26-weight build with every
-// grid letting its dependent start at once 1200 us, none of the larger ones 1130, when the others
-// were launched plainly; letting it before a CTA's write-out 951, as it ends 937).  A sampler only
-// waits: the test of the grid's size is 1 % of its instructions.  For an ordinary launch the
-// instructions do nothing.
-constexpr uint32_t kPdlMaxGrid = 2048;
+// (launch_pdl) may be scheduled as the last CTAs of the kernel before it in the stream end: its own
+// CTAs wait here until that kernel has completed and its memory is visible, so the launch and the CTAs'
+// start overlap the predecessor's tail instead of following it.  No kernel lets its dependent be
+// scheduled earlier (griddepcontrol.launch_dependents): CTAs that wait from early on take room from
+// those they wait for, and the split-pack's then run on SMs that keep the partition's large shared
+// memory and little L1.  Builds, us, with grids of up to 2048 CTAs releasing their dependents at once / none:
+// n = 10^6, split size 12, float-float 45 / 36; 2, compensated 43 / 36; n = 3.1 * 10^6 (757 partition
+// CTAs, all resident), 2, compensated 167 / 64; n = 2^22, 8, FP32 104 / 66; n = 8.38 * 10^6, 2, FP32 244 /
+// 195; n = 65,536 and below within 3 %.  Compensated ITS of 10^6 weights 29.6 / 24.3, Cutpoint 26.6 / 21.4.
+// For an ordinary launch the instruction does nothing.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-__device__ __forceinline__ void pdl_entry() {
-    pdl_wait();
-    if (gridDim.x <= kPdlMaxGrid) asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-}
 
 // Thread-block clusters.  arrive releases this thread's writes to the cluster's CTAs (shared and
 // global memory), wait acquires theirs; every thread of the cluster does both, in turn.

@@ -113,17 +113,16 @@ struct BatchView {
     int2* descent;               // per split-pack CTA: the shared top of its bisections
 };
 
-// Launches `kernel` (which starts with pdl_entry() or pdl_wait()) with programmatic stream
-// serialization: it may be scheduled before its predecessor in the stream has finished (when it has
-// let it be, or as its last CTAs end).  Measured against overlapping only grids of up to 2048 CTAs
-// (which then all let their dependents be scheduled at once): a 2^26-weight float-float build 972 ->
-// 937 us, a batch of 1024 distributions 772 -> 759 us, 512 served requests 1120 -> 1000 us, the small
-// configuration's pass 25.6 -> 25.5 us.
+// Launches `kernel` (which starts with pdl_wait()) with programmatic stream serialization: it may be
+// scheduled as its predecessor's last CTAs end.  Measured against overlapping only grids of up to 2048
+// CTAs: a 2^26-weight float-float build 972 -> 937 us, a batch of 1024 distributions 772 -> 759 us, 512
+// served requests 1120 -> 1000 us.
 //
 // overlap = false: an ordinary launch.  A grid of several waves that lives on the L1 (the alias sampler
 // on a table in L2) had better not begin on SMs whose shared memory a predecessor has claimed: the
 // split of L1 and shared memory changes only on an idle SM.  n = 4 x 10^6, 2^26 samples, right after the
 // split-pack: build and sampling 476 us overlapped, 401 not.
+constexpr uint32_t kOverlapMaxGrid = 2048;  // CTAs of such a sampler that are still overlapped
 template <class... KArgs, class... Args>
 inline cudaError_t launch_overlapped(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block,
                                      size_t smem, cudaStream_t st, Args&&... args) {

@@ -222,7 +222,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_alias_sample_batch(BatchView
 __global__ __launch_bounds__(kBlockBuildThreads, 8) void k_alias_blocks(
     const uint2* __restrict__ table, const uint32_t* __restrict__ classes, uint32_t n,
     AliasBlock* __restrict__ blocks, unsigned long long* __restrict__ reads) {
-    pdl_entry();
+    pdl_wait();
     __shared__ uint32_t s_sum[kBlockBuildThreads / 32];
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31u;
     const uint64_t base64 =
@@ -499,7 +499,7 @@ static_assert(kItsTreeLevels == static_cast<int>(kTreeTop), "shared levels above
 __global__ __launch_bounds__(kSampleThreads) void k_its_tree(const float* __restrict__ cmf,
                                                              uint32_t n, uint32_t L,
                                                              TreeBlock* __restrict__ blocks) {
-    pdl_entry();
+    pdl_wait();
     static_assert(its_tree_blocks(kTopBlockLevels) == kTopBlocks, "top block count");
     const size_t gb = static_cast<size_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if (gb >= its_tree_blocks(L)) return;
@@ -807,7 +807,7 @@ template <bool GRID>
 __global__ __launch_bounds__(kSampleThreads) void k_cell_groups(const float* __restrict__ cmf,
                                                                 uint32_t n, uint32_t G,
                                                                 uint32_t* __restrict__ group) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
     if (g < group_entries(G)) group[g] = group_start<GRID>(cmf, n, G, g);
 }
@@ -882,7 +882,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_cells(const float* __res
                                                               uint32_t n, uint32_t G,
                                                               const uint32_t* __restrict__ group,
                                                               ItsCell* __restrict__ cells) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
@@ -923,7 +923,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_grids(const float* __res
                                                               uint32_t n, uint32_t G,
                                                               const uint32_t* __restrict__ group,
                                                               ItsGrid* __restrict__ grids) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
@@ -1111,7 +1111,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_cmf_tile_min(const float* __
                                                                  uint32_t n,
                                                                  float* __restrict__ tile_min,
                                                                  uint32_t* __restrict__ bad) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float s_m[kSampleThreads / 32];
     const uint64_t base = static_cast<uint64_t>(blockIdx.x) * kTileItems;
     float m = INFINITY;
@@ -1138,7 +1138,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_cmf_tile_min(const float* __
 __global__ __launch_bounds__(1024) void k_tile_suffix_min(const float* __restrict__ tile_min,
                                                           uint32_t tiles,
                                                           float* __restrict__ suf) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float s_w[32];
     __shared__ float s_carry;
     if (threadIdx.x == 0) s_carry = INFINITY;
@@ -1197,7 +1197,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_cmf_mark(const float* __rest
                                                              uint32_t tiles,
                                                              ItsCell* __restrict__ cells,
                                                              uint32_t* __restrict__ bad) {
-    pdl_entry();
+    pdl_wait();
     __shared__ float s_w[kSampleThreads / 32];
     // one decision for the whole CTA (other CTAs may raise `bad` meanwhile)
     if (__syncthreads_or(*reinterpret_cast<volatile uint32_t*>(bad) != 0u)) return;
@@ -1236,7 +1236,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_cmf_mark(const float* __rest
 __global__ __launch_bounds__(kSampleThreads) void k_cells_mark_all(uint32_t G,
                                                                    ItsCell* __restrict__ cells,
                                                                    const uint32_t* __restrict__ bad) {
-    pdl_entry();
+    pdl_wait();
     if (*reinterpret_cast<const volatile uint32_t*>(bad) == 0u) return;
     for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < G; k += gridDim.x * blockDim.x)
         cells[k].y |= kCellUnsafe;
@@ -1385,7 +1385,7 @@ __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* 
                                                                    uint32_t n, uint32_t G,
                                                                    const uint32_t* __restrict__ group,
                                                                    uint32_t* __restrict__ guide) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t g = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;  // whole warps
     if (g * 32u >= G) return;
     uint32_t hi;
@@ -1487,7 +1487,7 @@ cudaError_t launch_its_sample_cells(cudaStream_t st, uint32_t rng, const float* 
 __global__ __launch_bounds__(kSampleThreads) void k_cutpoint_guide(const float* __restrict__ cmf,
                                                                    uint32_t n, uint32_t G,
                                                                    uint32_t* __restrict__ guide) {
-    pdl_entry();
+    pdl_wait();
     const uint32_t k = blockIdx.x * blockDim.x + threadIdx.x;
     if (k >= G) return;
     const float total = __ldg(cmf + n - 1u);
@@ -1682,7 +1682,7 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
     if (ctas > 0x7fffffffull) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(ctas));
     // (through the blocks it follows k_alias_blocks, which has no shared memory)
-    const bool overlap = b || ctas <= kPdlMaxGrid;
+    const bool overlap = b || ctas <= kOverlapMaxGrid;
     auto go = [&](auto kernel) {
         launch_overlapped(overlap, kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed,
                           offset, coop, out);
@@ -1714,7 +1714,7 @@ cudaError_t launch_batch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t co
                                       const BatchView& b) {
     if (b.sample_blocks == 0) return cudaSuccess;
     auto go = [&](auto kernel, uint32_t c) {
-        launch_overlapped(b.sample_blocks <= kPdlMaxGrid, kernel, b.sample_blocks, kSampleThreads, 0, st,
+        launch_overlapped(b.sample_blocks <= kOverlapMaxGrid, kernel, b.sample_blocks, kSampleThreads, 0, st,
                           b, c);
     };
     if (rng == RNG_REF) {

@@ -4,7 +4,7 @@ from __future__ import annotations
 
 import pytest
 
-from conftest import weights_uniform
+from conftest import weights_uniform, weights_zipf
 from gpu_util import h2d
 
 pytestmark = pytest.mark.gpu
@@ -37,3 +37,18 @@ def test_its_small_grid_is_not_slower(pkg, cuda):
         wrs.build(None, b, n)
         took[n] = _least_ms(cuda, lambda: wrs.sample(None, b, n, s, seed=1))
     assert took[1000] < 2.0 * took[65536], took
+
+
+def test_smaller_build_takes_less(pkg, cuda):
+    """Partitions of 757 and 1465 tiles against one of 2051: 0.38 and 0.73 of its time (0.99 and 1.1
+    when the smaller ones let the kernels after them start early)."""
+    W = pkg.wrs
+    cfg = W.AliasTableConfig(2)
+    wrs = W.WRS(cfg)
+    took = {}
+    for n in (3_100_003, 6_000_001, 8_400_003):
+        b = W.WRSBuffers.allocate(n, 1, cfg, handle=wrs.handle)
+        b.weights.copy_(h2d(weights_zipf(n, n)))
+        took[n] = _least_ms(cuda, lambda: wrs.build(None, b, n))
+    assert took[3_100_003] < 0.65 * took[8_400_003], took
+    assert took[6_000_001] < 0.92 * took[8_400_003], took
