@@ -117,15 +117,9 @@ struct BatchView {
 // scheduled as its predecessor's last CTAs end.  Measured against overlapping only grids of up to 2048
 // CTAs: a 2^26-weight float-float build 972 -> 937 us, a batch of 1024 distributions 772 -> 759 us, 512
 // served requests 1120 -> 1000 us.
-//
-// overlap = false: an ordinary launch.  A grid of several waves that lives on the L1 (the alias sampler
-// on a table in L2) had better not begin on SMs whose shared memory a predecessor has claimed: the
-// split of L1 and shared memory changes only on an idle SM.  n = 4 x 10^6, 2^26 samples, right after the
-// split-pack: build and sampling 476 us overlapped, 401 not.
-constexpr uint32_t kOverlapMaxGrid = 2048;  // CTAs of such a sampler that are still overlapped
 template <class... KArgs, class... Args>
-inline cudaError_t launch_overlapped(bool overlap, void (*kernel)(KArgs...), dim3 grid, dim3 block,
-                                     size_t smem, cudaStream_t st, Args&&... args) {
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                              cudaStream_t st, Args&&... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
@@ -135,13 +129,8 @@ inline cudaError_t launch_overlapped(bool overlap, void (*kernel)(KArgs...), dim
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = overlap ? 1 : 0;
+    cfg.numAttrs = 1;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Args&&>(args)...);
-}
-template <class... KArgs, class... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                              cudaStream_t st, Args&&... args) {
-    return launch_overlapped(true, kernel, grid, block, smem, st, static_cast<Args&&>(args)...);
 }
 // launch_pdl with clusters of `cluster` CTAs (at most 8)
 template <class... KArgs, class... Args>

@@ -1681,11 +1681,8 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
     if (ctas == 0) return cudaSuccess;
     if (ctas > 0x7fffffffull) return cudaErrorInvalidValue;
     const dim3 grid(static_cast<unsigned>(ctas));
-    // (through the blocks it follows k_alias_blocks, which has no shared memory)
-    const bool overlap = b || ctas <= kOverlapMaxGrid;
     auto go = [&](auto kernel) {
-        launch_overlapped(overlap, kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed,
-                          offset, coop, out);
+        launch_pdl(kernel, grid, kSampleThreads, 0, st, table, blocks, reads, n, S, seed, offset, coop, out);
     };
     if (rng == RNG_REF) {
         if (coop)
@@ -1714,8 +1711,7 @@ cudaError_t launch_batch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t co
                                       const BatchView& b) {
     if (b.sample_blocks == 0) return cudaSuccess;
     auto go = [&](auto kernel, uint32_t c) {
-        launch_overlapped(b.sample_blocks <= kOverlapMaxGrid, kernel, b.sample_blocks, kSampleThreads, 0, st,
-                          b, c);
+        launch_pdl(kernel, b.sample_blocks, kSampleThreads, 0, st, b, c);
     };
     if (rng == RNG_REF) {
         if (coop)
