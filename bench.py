@@ -134,12 +134,12 @@ def peaks() -> dict:
 def launches_per_step(n: int) -> int:
     """The library's kernel launches in one headline step (wrs_build + wrs_sample): total mass,
     partition, the split descent (split-pack grids of >= 512 CTAs of 479 subproblems), the
-    split-pack, the alias blocks (2^22 < N <= 2^26) and the sampler; up to eight tiles and 2048
+    split-pack, the alias blocks (5 * 2^20 < N <= 2^26) and the sampler; up to eight tiles and 2048
     subproblems, one build launch and the sampler."""
     if n <= 32768 and n // SPLIT_SIZE <= 2048:
         return 2
     blocks = -(-(n // SPLIT_SIZE) // 479)
-    return 4 + (blocks >= 512) + ((1 << 22) < n <= (1 << 26))
+    return 4 + (blocks >= 512) + ((5 << 20) < n <= (1 << 26))
 
 
 def profiled_traffic(l2_fetch: int, kernel: str = "coin_filter") -> float | None:

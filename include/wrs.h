@@ -181,7 +181,7 @@ void wrs_destroy(wrs_handle* h);
  * CMF above 2^16 weights they include the bisection's stored probe-tree blocks (at most ~2/7
  * of the CMF's bytes), which wrs_build writes and wrs_sample reads for the n built last; the
  * primitive wrs_its_sample probes the CMF alone (same samples).  For the alias method above
- * 2^22 weights they include the table's alias blocks and the partition's heavy bits (1 1/8 bytes
+ * 5 * 2^20 weights they include the table's alias blocks and the partition's heavy bits (1 1/8 bytes
  * per weight up to 2^26 in all): wrs_build writes them after the table and wrs_sample reads them for
  * the n built last, so that most samples skip the table read (same samples; wrs_split_pack and
  * wrs_pack into the buffers retire them until the next build, and the primitive wrs_alias_sample

@@ -248,10 +248,14 @@ cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint3
 // costs its 32-byte sector and the decoding (190 G samples/s while the blocks stay in L2); by the
 // table alone it costs its 8-byte entry, 250 G/s from L2 and 50 G/s from HBM.  2^26 samples of
 // uniform weights, us, by the table / through the blocks: n = 4.0 M 274 / 352, 6.0 M 423 / 353,
-// 8.0 M 549 / 353, 12 M 749 / 355; 2^28 samples: n = 2^26 5300 / 1640.  Beyond 2^26 the blocks no longer
-// fit L2.  The sampler reads the table alone when the blocks leave more than kBlockMaxReads eighths
+// 8.0 M 549 / 353, 12 M 749 / 355; 2^28 samples: n = 2^26 5300 / 1640, n = 2^27 5500 / 3100.  With the build
+// (whose blocks take 10-13), 2^26 samples: n = 4.25 M 377 / 446, Zipf 382 / 446; 5.0 M 444 / 456; 5.24 M 470 /
+// 460, Zipf 477 / 461; 2^24 samples 193 / 197 at 5.0 M and 203 / 200 at 5.24 M.  Above kBlockMaxN the blocks
+// would pay too; they end there because an index there takes more than the 26 bits of a block's head,
+// and the buffers' bytes and the launches of larger builds stay as they were without them.
+// The sampler reads the table alone when the blocks leave more than kBlockMaxReads eighths
 // of the samples to it (weights that the encoding does not fit: then a sample would pay for both).
-constexpr uint32_t kBlockMinN = 1u << 22;
+constexpr uint32_t kBlockMinN = 5u << 20;
 constexpr uint32_t kBlockMaxN = 1u << 26;
 constexpr uint32_t kBlockMaxReads = 6;
 // The non-cooperative ITS sampler's bisection probes one implicit binary tree (node k, root
