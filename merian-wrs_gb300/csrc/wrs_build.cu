@@ -171,7 +171,6 @@ __global__ __launch_bounds__(kTileThreads) void k_total_mass(const float* __rest
         ctrl->mean = m.hi;
         ctrl->mean_lo = m.lo;
         ctrl->mass_done = 0u;
-        ctrl->block_reads = 0ull;  // the alias blocks of this build add to it
     }
 }
 
@@ -521,9 +520,12 @@ __device__ __forceinline__ void partition_tile(const PartArgs& a, const BatchVie
         }
         const uint32_t tc = __popc(heavies);
         if constexpr (!BATCH && CARRY == Carry::kLookback) {
-            if (a.classes)
+            if (a.classes) {
                 a.classes[static_cast<size_t>(lt) * kTileThreads + threadIdx.x] =
                     static_cast<uint16_t>(heavies);
+                // (a build whose alias blocks follow: they add to it)
+                if (lt == 0u && threadIdx.x == 0) ctrl->block_reads = 0ull;
+            }
         }
         const uint32_t ic = warp_incl_u(tc, lane);
         s_lc[threadIdx.x] = ic - tc;
@@ -2285,7 +2287,6 @@ __global__ __launch_bounds__(kTileThreads, 1) void k_build_small(PartArgs a, Spl
                 a.ctrl->mean64 = m.m64;
                 a.ctrl->mean = m.hi;
                 a.ctrl->mean_lo = m.lo;
-                a.ctrl->block_reads = 0ull;
             }
         }
     }

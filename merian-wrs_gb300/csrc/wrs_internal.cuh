@@ -240,7 +240,7 @@ cudaError_t launch_alias_sample(cudaStream_t st, uint32_t rng, uint32_t coop, co
                                 const AliasBlock* blocks, const unsigned long long* reads,
                                 uint32_t n, uint64_t s, uint64_t seed, uint64_t offset,
                                 uint32_t* out);
-// the blocks of table[0, n) and, into *reads (zero: k_total_mass clears it), 8 times the entry
+// the blocks of table[0, n) and, into *reads (zero: the build's partition clears it), 8 times the entry
 // reads one sample of every bucket would cost; classes: the partition's heavy bits
 cudaError_t launch_alias_blocks(cudaStream_t st, const uint2* table, const uint32_t* classes,
                                 uint32_t n, AliasBlock* blocks, unsigned long long* reads);
