@@ -726,7 +726,9 @@ __global__ __launch_bounds__(kSampleThreads) void k_its_sample_tree(const float*
 __device__ __forceinline__ int its_shift(float total, uint32_t G) {
     const uint32_t e = __float_as_uint(total) >> 23;
     if (e == 0u) return 127;           // zero or denormal: F < 2^(127 - 126) steps
-    if (e >= 255u) return 7;           // not finite (or negative): results are meaningless
+    // infinite (the weights' sum exceeds FP32's range): finite values are below 4 steps, all in cell 0,
+    // the others start at the first infinite one (NaN or negative: results are meaningless)
+    if (e >= 255u) return -126;
     const int E = 31 - __clz(static_cast<int>(G));
     // total = m 2^(e - 127), 1 <= m < 2: total * 2^s / 128 = m 2^E or half of it
     const float m = __uint_as_float((__float_as_uint(total) & 0x7fffffu) | 0x3f800000u);
@@ -741,7 +743,7 @@ __device__ __forceinline__ float pow2f(int e) {
 template <bool GRID>
 __device__ __forceinline__ float cell_step(const float* __restrict__ cmf, uint32_t n, uint32_t G) {
     const float total = __ldg(cmf + n - 1u);
-    if constexpr (GRID) return pow2f(7 - its_shift(total, G));  // (unused for G = 1)
+    if constexpr (GRID) return pow2f(min(7 - its_shift(total, G), 128));  // (2^128: infinite)
     return __fdiv_rn(total, __uint2float_rn(G));
 }
 // threshold c_k of cell k

@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 
 from conftest import weights_lognormal, weights_precision, weights_uniform, weights_zipf
-from gpu_util import h2d
+from gpu_util import d2h, h2d
 
 pytestmark = pytest.mark.gpu
 
@@ -71,3 +71,29 @@ def test_grid_around_the_cached_size(pkg, cuda, n, rng):
         wrs.its_sample(None, b.internals.views()["cmf"], n, s, 9, 0, out[1].data_ptr())
         cuda.cuda.synchronize()
         assert cuda.equal(out[0], out[1])
+
+
+@pytest.mark.parametrize("rng", [0, 1])
+@pytest.mark.parametrize("entry", [1, 4, 40, 20_000])  # the last: one cell
+def test_infinite_total(pkg, cuda, entry, rng):
+    """Finite weights whose sum exceeds FP32's range (no tile's does): the CMF ends in infinities, the
+    Philox stream's targets spread over the finite values all the same."""
+    W = pkg.wrs
+    n = 6 * 4096 + 17
+    w = weights_uniform(n, 3)
+    w[7::4096] = 1e38
+    cfg = W.ITSConfig(guiding_entry_size=entry, rng=rng, scan_precision=W.SCAN_COMPENSATED)
+    wrs = W.WRS(cfg)
+    b = W.WRSBuffers.allocate(n, 1, cfg, handle=wrs.handle)
+    b.weights.copy_(h2d(w))
+    wrs.build(None, b, n)
+    cmf = d2h(b.internals.views()["cmf"], n, np.float32)
+    assert np.isinf(cmf[-1]) and np.isfinite(cmf[3 * 4096 + 6]) and np.isinf(cmf[3 * 4096 + 7])
+    s = 100_001
+    out = cuda.full((2, s), -1, dtype=cuda.int32, device="cuda")
+    W.check(W.lib().wrs_sample_at(wrs.handle.ptr, None, b.internals.ptr, n, s, 9, 0,
+                                  out[0].data_ptr()))
+    wrs.its_sample(None, b.internals.views()["cmf"], n, s, 9, 0, out[1].data_ptr())
+    cuda.cuda.synchronize()
+    assert cuda.equal(out[0], out[1])
+    assert rng == 0 or len(out[0].unique()) >= 4
