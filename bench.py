@@ -1,5 +1,6 @@
 #!/usr/bin/env python3
-"""Benchmark of the WRS hot path on GB300 (one JSON line on stdout, rank 0).
+"""Benchmark of the WRS hot path on GB300 (one JSON line on stdout, rank 0: the headline; the full
+line, with every configuration, goes to stderr).
 
 Workload (the single-large-distribution configuration): N = 2^26 FP32 weights in three
 seeded distributions -- uniform(0,1], Zipf-like (i+1)^-1.1 randomly permuted, log-normal
@@ -16,7 +17,7 @@ needed between steps.
           index) / its mean CUDA-event duration, against the measured HBM copy bandwidth
   cpu_baseline  the CPU port of the same path (oracle/, single thread) on a bounded sample
 
-Extra keys measure the rest of the configuration with the same events: per-kernel times
+Extra keys of the full line measure the rest of the configuration with the same events: per-kernel times
 and bandwidths, the decoupled scan (weights scanned/s) and ITS sampling (samples/s); and
 "batched", the mixed-size configuration (4096 distributions, N log-uniform in [64, 2^20],
 2^30 samples in total) as one CUDA graph against 4096 per-call build + sample pairs; and
@@ -641,9 +642,29 @@ def main() -> None:
             "scan_and_its": cpu_scan_its(w0, nthreads),
             "reference_cpu": reference_cpu(w0)}
     if rank == 0:
-        print(json.dumps(line), flush=True)
+        print(json.dumps(line), file=sys.stderr, flush=True)
+        print(json.dumps(headline_line(line)), flush=True)
     if dist is not None:
         dist.destroy_process_group()
+
+
+# keys of the full line that the headline line leaves out, and what it keeps of the long ones
+DETAIL_KEYS = ("statistics", "per_distribution", "kernels", "batched", "served", "small", "precision")
+HEADLINE_PARTS = {
+    "autotune": ("l2_fetch",),
+    "e2e": ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step", "passes_samples_per_s",
+            "kernel_to_host_value", "serial_value"),
+    "roofline": ("bound", "achieved", "peak", "unit", "frac", "traffic", "kernel", "peak_source"),
+    "cpu_baseline": ("value", "unit", "cores", "kind"),
+}
+
+
+def headline_line(line: dict) -> dict:
+    """What the benchmark prints on stdout: the headline of the full line (which goes to stderr with
+    every configuration, some 26 KB), short enough for a log that keeps the last few KB."""
+    return {key: {k: value[k] for k in HEADLINE_PARTS[key] if k in value}
+            if key in HEADLINE_PARTS else value
+            for key, value in line.items() if key not in DETAIL_KEYS}
 
 
 BATCH_DISTS = 4096

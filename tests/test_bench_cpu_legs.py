@@ -104,3 +104,53 @@ def test_launches_per_step():
     assert bench.launches_per_step(1 << 26) == 6
     assert bench.launches_per_step((1 << 26) + 5) == 5
     assert bench.launches_per_step(65536) == 4
+
+
+def test_headline_line_is_short_and_whole():
+    """The line on stdout fits a log's last 3 KB and holds the keys a reader of the headline needs,
+    whatever the configurations add to the full line."""
+    import json
+    import bench
+    text = "x" * 600
+    line = {
+        "metric": bench.METRIC, "value": 9.87654321e10, "unit": "samples/s", "n_gpus": 1, "steps": 20,
+        "warmup": 5, "ms_per_step": 2.7212345678, "higher_is_better": True, "scaling": "weak",
+        "vs_baseline": None, "dtype": "f32", "data": "synthetic (seeded)",
+        "config": bench.headline_config(1 << bench.LOG2_N, 1 << bench.LOG2_S, 1),
+        "autotune": {"l2_fetch": 64, "trials": [{"ms": 1.0}] * 3, "method": text},
+        "e2e": {"value": 4.14e10, "unit": "samples/s", "h2d_bytes_per_step": 1 << 28,
+                "d2h_bytes_per_step": 1 << 30, "method": text,
+                "passes_samples_per_s": [4.1234567891e10] * bench.E2E_PASSES,
+                "kernel_to_host_value": 3.681234e10, "serial_value": 2.1234e10,
+                "host_link": {"h2d": 2.1e11, "d2h": 1.93e11}},
+        "roofline": {"bound": "hbm", "achieved": 1950.123456, "peak": 6782.8, "unit": "GB/s",
+                     "frac": 0.2875, "traffic": 5605270000.0, "traffic_source": text,
+                     "kernel": "k_alias_sample", "bytes_model": text, "peak_source": "measured",
+                     "random_gather": {"rate": 6e10, "model": text}},
+        "alias_builds_per_s": 1050.123456789, "build_ms_mean": 0.9512345678,
+        "sample_ms_mean": 1.7012345678,
+        "clocks": {"sm_mhz": 2070.0, "sm_max_mhz": 2070.0, "reasons": ["sw_power_cap"],
+                   "samples": 20, "power_w_max": 782.42},
+        "gpu_launches": 120, "device_status": {"timeout": False, "split_overlap_beyond_window": False},
+        "cpu_baseline": {"value": 6.9e7, "unit": "samples/s", "cores": 16, "kind": "port",
+                         "sample": text, "scan_and_its": {"sample": text}},
+        **{key: {"rows": [text] * 8} for key in bench.DETAIL_KEYS},
+    }
+    short = bench.headline_line(line)
+    assert len(json.dumps(short)) < 2600
+    for key in ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step",
+                "higher_is_better", "scaling", "vs_baseline", "dtype", "data", "config", "clocks",
+                "gpu_launches"):
+        assert short[key] == line[key]
+    for key in ("value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step"):
+        assert short["e2e"][key] == line["e2e"][key]
+    assert not set(short) & set(bench.DETAIL_KEYS)
+
+
+def test_traffic_of_the_sampler_in_use():
+    """The roofline names the sampler through the alias blocks: 5.6 GB a launch at 64 bytes, 8.4 at 128,
+    nothing where nothing was captured."""
+    import bench
+    assert bench.profiled_traffic(64, "blocks") == 5605270000
+    assert bench.profiled_traffic(128, "blocks") == 8403100000
+    assert bench.profiled_traffic(32, "blocks") is None
