@@ -36,3 +36,24 @@ def test_groups_equal_the_bisection(pkg, cuda, n, entry, gen, rng, rest):
     cuda.cuda.synchronize()
     assert cuda.equal(out[0], out[1])
     assert int(out[0].min()) >= 0 and int(out[0].max()) < n
+
+
+@pytest.mark.parametrize("rng", [0, 1])
+@pytest.mark.parametrize("entry", [32, 400])
+def test_infinite_total(pkg, cuda, entry, rng):
+    """Finite weights whose sum exceeds FP32's range: ranges that end in an infinite value."""
+    W = pkg.wrs
+    n, s = 6 * 4096 + 17, 1 << 19
+    w = weights_uniform(n, 3)
+    w[7::4096] = 1e38
+    cfg = W.CutpointConfig(entry, rng=rng, scan_precision=W.SCAN_COMPENSATED)
+    wrs = W.WRS(cfg)
+    b = W.WRSBuffers.allocate(n, s, cfg, handle=wrs.handle)
+    b.weights.copy_(h2d(w))
+    wrs.build(None, b, n)
+    v = b.internals.views()
+    wrs.sample(None, b, n, s, seed=3)
+    ref = cuda.empty_like(b.samples)
+    wrs.cutpoint_sample(None, v["cmf"], n, v["guide_table"], s, 3, 0, ref.data_ptr())
+    cuda.cuda.synchronize()
+    assert cuda.equal(b.samples, ref)
