@@ -13,7 +13,8 @@
 //   3. launch -- wrs_batch_set / wrs_batch_build / (cross-slot waits) / wrs_batch_sample on
 //                the slot's stream, then the device status word is copied back and the
 //                slot's completion event recorded.
-// Slots run on separate non-blocking streams, so a new batch overlaps with those in flight.
+// Slots run on separate non-blocking streams, so a new batch overlaps with those in flight; one much
+// smaller than they are runs at the greater priority.
 #include <algorithm>
 #include <chrono>
 #include <cstring>
@@ -124,7 +125,9 @@ struct InFlight {
 };
 
 struct Slot {
-    cudaStream_t stream = nullptr;
+    cudaStream_t stream = nullptr;            // the one of `streams` that its batch in flight uses
+    cudaStream_t streams[2] = {nullptr, nullptr};  // of the least and the greatest priority
+    uint64_t weights = 0;                     // that its batch in flight builds from
     cudaEvent_t done = nullptr;
     wrs_batch* batch = nullptr;
     uint32_t* status_host = nullptr;  // pinned copy of the batch's device status word
@@ -309,6 +312,14 @@ wrs_status admit_and_launch(wrs_server* s, size_t k, bool& launched) {
         s->queue.pop_front();
     }
     if (descs.empty()) return WRS_OK;
+    // A batch much smaller than one in flight goes ahead of it: its kernels, which fill little of the
+    // chip, then run beside the larger one's and not after them.  A burst of 512 requests (batches of 406
+    // and 106): 1058 us by one priority, 943 so.  Below half, so that equal batches share the chip.
+    sl.weights = weights;
+    uint64_t ahead = 0;
+    for (const Slot& o : s->slots)
+        if (o.busy) ahead = std::max(ahead, o.weights);
+    sl.stream = sl.streams[2u * weights < ahead ? 1 : 0];
     wrs_status st = wrs_batch_set(sl.batch, sl.stream, descs.data(),
                                   static_cast<uint32_t>(descs.size()));
     if (st == WRS_OK) st = wrs_batch_build(s->h, sl.stream, sl.batch);
@@ -340,10 +351,12 @@ uint32_t take_completions(wrs_server* s, wrs_completion* out, uint32_t max_out) 
 
 void destroy_slots(wrs_server* s) {
     for (Slot& sl : s->slots) {
-        if (sl.stream) cudaStreamSynchronize(sl.stream);
+        for (cudaStream_t q : sl.streams)
+            if (q) cudaStreamSynchronize(q);
         if (sl.batch) wrs_batch_destroy(sl.batch);
         if (sl.done) cudaEventDestroy(sl.done);
-        if (sl.stream) cudaStreamDestroy(sl.stream);
+        for (cudaStream_t q : sl.streams)
+            if (q) cudaStreamDestroy(q);
         if (sl.status_host) cudaFreeHost(sl.status_host);
     }
     s->slots.clear();
@@ -395,7 +408,11 @@ wrs_status wrs_server_create(const wrs_handle* h, const wrs_server_config* c, wr
         wrs_status st = wrs_batch_create(h, c->max_batch_dists, c->max_batch_weights,
                                          c->max_batch_samples, &sl.batch);
         if (st == WRS_OK) {
-            e = cudaStreamCreateWithFlags(&sl.stream, cudaStreamNonBlocking);
+            int least = 0, greatest = 0;
+            e = cudaDeviceGetStreamPriorityRange(&least, &greatest);
+            for (int q = 0; q < 2 && e == cudaSuccess; ++q)
+                e = cudaStreamCreateWithPriority(&sl.streams[q], cudaStreamNonBlocking,
+                                                 q ? greatest : least);
             if (e == cudaSuccess) e = cudaEventCreateWithFlags(&sl.done, cudaEventDisableTiming);
             if (e == cudaSuccess)
                 e = cudaHostAlloc(reinterpret_cast<void**>(&sl.status_host), sizeof(uint32_t),
