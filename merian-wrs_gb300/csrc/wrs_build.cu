@@ -2231,8 +2231,8 @@ __global__ __launch_bounds__(kSplitThreads, 4) void k_split_pack(SplitArgs a, Ba
 // carries are exact, or added tile by tile in FP32 mode).  The subproblems are shared out evenly; every
 // load waits alone here, so bisections read three levels at a time and the walks' weights come through
 // shared memory.  Builds one after the other, three launches -> this one: n = 1000, split size 2, FP32
-// 12.2 -> 9.0 us; n = 4096, 12, float-float 18.2 -> 14.8; n = 16384, 12, float-float 23.0 -> 17.4; n =
-// 32768, 32, float-float 48 -> 22.  At n = 1000 the load and the mass take 2 us of it, mean and
+// 11.4 -> 8.7 us; n = 4096, 12, float-float 19.9 -> 14.6; n = 16384, 12, float-float 24.3 -> 17.8; n =
+// 32768, 16, float-float 26.8 -> 22.7, 32, compensated 49.2 -> 17.6.  At n = 1000 the load and the mass take 2 us of it, mean and
 // partition 3.4, splits 1.8, walks and write-out 1.9.
 constexpr uint32_t kSmallCtas = 8;
 constexpr uint32_t kSmallPack = kTileThreads;  // subproblems per CTA, at most: one per thread

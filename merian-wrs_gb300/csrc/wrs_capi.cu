@@ -3,19 +3,23 @@
 // The handle holds the configuration (the reference's WRSConfig variant); a buffers
 // object holds the internals of one distribution (the reference's WRSBuffers minus the
 // caller-owned weights and samples) in a single device allocation.  Launch sequences:
-//   alias build : k_total_mass -> k_prefix_partition -> k_split_pack
+//   alias build : k_total_mass -> k_prefix_partition -> (k_split_descent ->) k_split_pack, above
+//                 kBlockMinN weights -> k_alias_blocks; k_build_small for a small distribution
 //                 (PSA::run, src/device/wrs/alias/psa/PSA.hpp:170-237)
 //   ITS build   : k_scan_bulk, or k_total_mass -> k_scan_exact in the compensated precisions
-//                 (ITS::build, src/device/wrs/its/ITS.hpp:90-108), then with a cell size
-//                 k_its_cells (the cell blocks k_its_sample_cells reads); on the FP32 CMF also
-//                 the cell marks (k_cmf_tile_min -> k_tile_suffix_min -> k_cmf_mark) and
-//                 k_its_tree (the probe-tree blocks the marked cells and cell size 0 bisect in)
-//   Cutpoint    : the same scan -> k_cutpoint_guide, or k_guide_monotone on the compensated CMF
-//                 (Cutpoint::build, src/device/wrs/cutpoint/Cutpoint.hpp:108-138)
-//   sample      : k_alias_sample | k_its_sample (k_its_sample_cells) | k_cutpoint_sample
+//                 (ITS::build, src/device/wrs/its/ITS.hpp:90-108), then with a cell size, and
+//                 (k_cell_groups ->) before each: the compensated CMF's grid, k_its_grids (which
+//                 k_its_sample_grids reads); the FP32 CMF's cells, k_its_cells (which
+//                 k_its_sample_cells reads), with their marks (k_cmf_tile_min ->
+//                 k_tile_suffix_min -> k_cmf_mark) and k_its_tree (the probe-tree blocks the
+//                 marked cells and cell size 0 bisect in)
+//   Cutpoint    : the same scan -> k_cutpoint_guide, or (k_cell_groups ->) k_guide_monotone on the
+//                 compensated CMF (Cutpoint::build, src/device/wrs/cutpoint/Cutpoint.hpp:108-138)
+//   sample      : k_alias_sample | k_its_sample (_grids, _cells, _tree) | k_cutpoint_sample (_mono)
 //                 (WRS::sample, src/device/wrs/WRS.hpp:145-168)
-//   batch       : k_batch_maps (wrs_batch_set), then the same three build kernels and the
-//                 alias sampler over all distributions of a batch, one launch each
+//   batch       : k_batch_maps (wrs_batch_set), then k_total_mass, k_prefix_partition,
+//                 k_split_descent, k_split_pack and the alias sampler over all distributions of
+//                 a batch, one launch each
 // Stream order replaces the reference's pipeline barriers.
 #include <cstdio>
 #include <cstring>
@@ -141,8 +145,8 @@ Layout layout_for(const wrs_config& cfg, uint32_t max_n) {
                         : 0;
     } else {
         L.cmf = take(sizeof(float) * static_cast<size_t>(max_n));
-        // Cutpoint: its guiding table; ITS: the cell blocks that steer sampling (none with
-        // guiding_entry_size 0) and their construction scratch
+        // Cutpoint: its guiding table; ITS: the cells or the grid that steer sampling (none with
+        // guiding_entry_size 0); the construction scratch of either
         const uint32_t G = cfg.guiding_entry_size ? guide_entries(max_n, cfg.guiding_entry_size) : 0;
         const bool its = cfg.method == WRS_METHOD_ITS;
         if (!its)
@@ -369,7 +373,7 @@ static bool its_guided(const wrs_handle* h) {
     return h->cfg.method == WRS_METHOD_ITS && h->cfg.coop_size == 0 &&
            h->cfg.guiding_entry_size != 0;
 }
-// the guiding table / cell blocks the handle will use exist in b and have its size
+// the guiding table, cells or grid that the handle will use exist in b and have its size
 static wrs_status check_tables(const wrs_handle* h, const wrs_buffers* b) {
     if ((h->cfg.method == WRS_METHOD_CUTPOINT || its_guided(h)) &&
         b->cfg.guiding_entry_size != h->cfg.guiding_entry_size)
@@ -562,8 +566,8 @@ wrs_status wrs_build(const wrs_handle* h, void* stream, const float* weights, ui
         WRS_CUDA(launch_scan(st, comp, weights, n, b->cmf, b->ctrl, b->scan_states, b->cap_tiles,
                              b->partials),
                  "ITS build");
-        // the compensated CMF is exactly non-decreasing: the galloping construction gives
-        // the bisection's entries
+        // the compensated CMF is exactly non-decreasing: searches inside brackets give the
+        // bisection's entries
         const uint32_t G = guide_entries(n, h->cfg.guiding_entry_size);
         if (comp) b->monotone_n = n;
         if (h->cfg.method == WRS_METHOD_CUTPOINT)

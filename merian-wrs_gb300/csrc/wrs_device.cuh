@@ -396,7 +396,7 @@ __device__ __forceinline__ uint2 ld_entry_policy(const uint2* p, uint64_t pol) {
 }
 
 // An L2 eviction policy (createpolicy) and read-only loads that carry it: data read once at
-// random (a large CMF, the ITS cell blocks) is marked evict-first.
+// random (a large CMF, the FP32 CMF's cells) is marked evict-first.
 __device__ __forceinline__ uint64_t l2_policy_evict_first() {
     uint64_t p;
     asm("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(p));

@@ -331,7 +331,7 @@ cudaError_t launch_its_sample_cells(cudaStream_t st, uint32_t rng, const float* 
                                     uint32_t L);
 // ITS on the compensated (exactly non-decreasing) CMF: F(v) = floor(v * 2^s) cuts the CMF's values
 // into cells of 128 steps, the power 2^s such that at most its_grids(n, entry) cells hold them
-// (its_scale).  Cell k = F >> 7 is one 32-byte sector: the first index x with F(cmf[x]) >= 128 k and,
+// (its_shift).  Cell k = F >> 7 is one 32-byte sector: the first index x with F(cmf[x]) >= 128 k and,
 // for up to kGridSlots parts of 2^e items from x on, the step (7 bits) of each part's last item.
 // The product is exact and F monotone, so an item of a lower step than a target's is below it and
 // one of a higher step is not, and of equal steps >= 2^23 (where values are whole steps) neither is

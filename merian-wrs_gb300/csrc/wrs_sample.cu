@@ -84,9 +84,10 @@ __device__ __forceinline__ BlockSays block_says(const uint4& lo, const uint4& hi
 // By the table alone a sample is one random 8-byte read: from a table beyond L2 the device's rate of
 // random HBM accesses bounds it (50-70 G/s, whatever the bytes), from one in L2 the L1's one
 // wavefront per gathered sector (250 G/s).  Through the blocks (1 byte per bucket: 64 MB at n = 2^26,
-// mostly in L2) one 32-byte sector decides 86 % of uniform weights' samples and the bound is
-// instruction issue (72 % active, ~150 instructions per 32 samples; 22 % of the blocks still miss
-// L2 at 2^26): 2^28 samples, n = 2^26, uniform 2.76 -> 1.64 ms, log-normal(0, 2) 4.3 -> 1.73; 2 x 10^8
+// 22 % of whose reads miss L2 there) one 32-byte sector decides 86 % of uniform weights' samples.  The
+// bounds are instruction issue (72 % active, ~150 instructions per 32 samples) and, at 2^26, the random
+// accesses of block misses and entries together (16 bytes read from HBM a sample in fetches of 64: 40
+// G/s): 2^28 samples, n = 2^26, uniform 2.76 -> 1.64 ms, log-normal(0, 2) 4.3 -> 1.73; 2 x 10^8
 // samples, n = 5 x 10^7, Zipf 3.3 -> 1.10 ms (against one byte of p per bucket, which decided only the
 // samples that their bucket keeps).
 template <uint32_t RNG, bool COOP, bool BLOCKS, int PT = kAliasPerThread>
