@@ -2417,6 +2417,10 @@ static void split_dispatch(cudaStream_t st, bool r64, bool ff, uint32_t grid, co
         launch_split_kernel<false, false, BATCH, false>(st, grid, a, bv);
 }
 
+// Split-pack CTAs from which the shared descent has a launch of its own.  Builds, with it / without: 522
+// CTAs (n = 10^6, split size 4, float-float, Zipf) 39 / 34 us, 783 (6 x 10^6, 16, compensated) 117 / 128, (3 x
+// 10^6, 8, FP32) 52 / 49, 1566 (3 x 10^6, 4, float-float) 66 / 68, 3132 62 / 70, 3915 (3 x 10^7, 16) 419 / 469:
+// it pays for certain from about 1500 on, by weights and precision from 700.
 constexpr uint32_t kDescentMinBlocks = 512;
 
 cudaError_t launch_split_pack(cudaStream_t st, bool r64, bool full_light, const float* w,

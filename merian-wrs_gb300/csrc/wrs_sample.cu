@@ -1399,8 +1399,9 @@ __global__ __launch_bounds__(kSampleThreads) void k_guide_monotone(const float* 
 
 // Up to this many cells the second pass's warps find their brackets themselves: a launch less, and
 // few enough warps that all wait at once.  Builds, with the first pass / without: ITS n = 65536 (8192
-// cells) 26.5 / 24.2 us, n = 5000 22.6 / 20.9, n = 4 x 10^6 (500 K) 53.3 / 57.2; Cutpoint, entry 32, n =
-// 10^5 (3125) 25.2 / 24.3, n = 2^22 (131072) 44.3 / 47.4.
+// cells) 18.6 / 16.7 us, n = 5000 14.8 / 13.9, n = 262144 (32768) 19.6 / 17.4; Cutpoint, entry 32, n = 10^5
+// (3125) 18.1 / 16.9, n = 10^6 (31250) 23.3 / 21.3.  The line is where both met when kernels still let their
+// dependents start early; since then n = 2^22 (131072) takes 34.6 / 32.3, so it is on the safe side.
 constexpr uint32_t kOwnMaxCells = 32768;
 
 // the first pass (group: group_entries(G) words); true: left to the second
